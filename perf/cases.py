@@ -12,6 +12,7 @@ so that a state is a few GB.
   run(state)          one pass; returns what the pass computes
   work(case)          bytes and operations the pass cannot do without
   tolerance(case)     how far another correct implementation of the same precision may be off
+  exact(case, seed)   what run returns, in 64 bits and plain torch
 """
 import os
 import socket
@@ -298,3 +299,130 @@ _TOLERANCE = {"train": (0.03, 0.99), "logits": (0.03, 0.25), "attention": (0.013
 def tolerance(case):
     rel, most = _TOLERANCE[case["kind"]]
     return {"rel": rel, "max": most}
+
+
+# ---- the same passes in 64 bits, in plain torch ---------------------------------------------------------------------------
+def _rms_norm(x, weight, eps=1e-5):
+    return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * weight
+
+
+def _rotate(x, dim):
+    """Rotary embedding of the last axis of [s, b, heads, dim], halves rotated."""
+    inv = 1.0 / (10000.0 ** (torch.arange(0, dim, 2, dtype=torch.float32, device=x.device) / dim))
+    angle = torch.outer(torch.arange(x.shape[0], dtype=torch.float32, device=x.device), inv).double()
+    cos, sin = (torch.cat((f, f), -1)[:, None, None, :] for f in (angle.cos(), angle.sin()))
+    a, b = x.chunk(2, -1)
+    return x * cos + torch.cat((-b, a), -1) * sin
+
+
+def _one_head(q, k, v, causal):
+    s = q @ k.t() / q.shape[1] ** 0.5
+    if causal:
+        s = s.masked_fill(torch.ones_like(s, dtype=torch.bool).triu(1 + k.shape[0] - q.shape[0]), float("-inf"))
+    return s.softmax(-1) @ v
+
+
+def _attention(q, k, v, causal):
+    """[s, b, heads, d], a head at a time and its scores formed again in backward."""
+    from torch.utils.checkpoint import checkpoint
+    rep = q.shape[2] // k.shape[2]
+    out = [torch.stack([checkpoint(_one_head, q[:, i, h], k[:, i, h // rep], v[:, i, h // rep], causal, use_reentrant=False)
+                        for h in range(q.shape[2])], 1) for i in range(q.shape[1])]
+    return torch.stack(out, 1)
+
+
+def _swiglu(x):
+    a, b = x.chunk(2, -1)
+    return torch.nn.functional.silu(a) * b
+
+
+def _logits(c, w, tokens):
+    """tokens [b, s] -> [b, s, vocab]; w: the model's weights by name."""
+    x = w["embedding.word_embeddings.weight"][tokens.t()]
+    heads, kv = c["heads"], c["kv"]
+    for i in range(c["layers"]):
+        p = "decoder.layers.%d." % i
+        h = _rms_norm(x, w[p + "input_layernorm.weight"]) @ w[p + "self_attention.linear_qkv.weight"].t()
+        h = h.view(*h.shape[:2], kv, heads // kv + 2, D)
+        q, k, v = h[..., :-2, :].reshape(*h.shape[:2], heads, D), h[..., -2, :], h[..., -1, :]
+        x = x + _attention(_rotate(q, D), _rotate(k, D), v, True).flatten(2) @ w[p + "self_attention.linear_proj.weight"].t()
+        h = _rms_norm(x, w[p + "pre_mlp_layernorm.weight"]) @ w[p + "mlp.linear_fc1.weight"].t()
+        x = x + _swiglu(h) @ w[p + "mlp.linear_fc2.weight"].t()
+    return (_rms_norm(x, w["decoder.final_layernorm.weight"]) @ w["output_layer.weight"].t()).transpose(0, 1)
+
+
+def _experts(c, w, x):
+    flat = x.reshape(-1, x.shape[-1])
+    n, e = flat.shape[0], c["experts"]
+    logits = flat @ w["router.weight"].t()
+    if c["score"] == "softmax":
+        top, idx = logits.topk(c["topk"], 1)
+        top, scores = top.softmax(-1), logits.softmax(-1)
+    else:
+        top, idx = logits.sigmoid().topk(c["topk"], 1)
+        scores = logits.sigmoid()
+        top, scores = top / top.sum(-1, keepdim=True), scores / scores.sum(-1, keepdim=True)
+    chosen = torch.zeros_like(logits).scatter(1, idx, 1.0)
+    if c["score"] == "softmax":
+        balance = (scores.sum(0) * chosen.sum(0)).sum() * (e * 0.01 / (n * n * c["topk"]))
+    else:
+        per = (scores.view(c["seq"], c["b"], e).sum(0) * chosen.view(c["seq"], c["b"], e).sum(0)).sum()
+        balance = per * (e * 0.0001 / (c["seq"] ** 2 * c["topk"] * c["b"]))
+    out = torch.zeros_like(flat)
+    for i in range(e):
+        row, slot = (idx == i).nonzero(as_tuple=True)
+        out = out.index_add(0, row, _swiglu(flat[row] @ w["experts.weight1"][i]) @ w["experts.weight2"][i] * top[row, slot, None])
+    if c["shared"]:
+        out = out + _swiglu(flat @ w["shared_experts.linear_fc1.weight"].t()) @ w["shared_experts.linear_fc2.weight"].t()
+    return out.view_as(x), balance
+
+
+def _latent_attention(c, w, x):
+    n, qk = c["heads"], QK_NOPE + QK_ROPE
+    q = _rms_norm(x @ w["linear_q_down_proj.weight"].t(), w["q_layernorm.weight"]) @ w["linear_q_up_proj.weight"].t()
+    q = q.view(*x.shape[:2], n, qk)
+    low, k_pe = (x @ w["linear_kv_down_proj.weight"].t()).split([KV_LORA, QK_ROPE], -1)
+    kv = (_rms_norm(low, w["kv_layernorm.weight"]) @ w["linear_kv_up_proj.weight"].t()).view(*x.shape[:2], n, QK_NOPE + V_DIM)
+    k_pe = _rotate(k_pe[:, :, None], QK_ROPE).expand(-1, -1, n, -1)
+    q = torch.cat((q[..., :QK_NOPE], _rotate(q[..., QK_NOPE:], QK_ROPE)), -1)
+    k = torch.cat((kv[..., :QK_NOPE], k_pe), -1)
+    return _attention(q, k, kv[..., QK_NOPE:], True).flatten(2) @ w["linear_proj.weight"].t()
+
+
+def exact(case, seed):
+    """What ``run`` returns on the state of ``prepare(case, seed)``, in 64 bits.  The fp8 layer is given without its rounding of
+    the operands; the weights after an optimizer step have no such value (their first update is little more than the sign of a
+    gradient)."""
+    c = dict(case)
+    st = prepare(case, seed)
+    kind = c["kind"]
+    if kind == "attention":
+        q, k, v = (st[n].detach().double().requires_grad_(True) for n in "qkv")
+        out = _attention(q, k, v, c["causal"])
+        return dict(zip(("out", "dq", "dk", "dv"), (out.detach(),) + torch.autograd.grad(out, (q, k, v), st["dout"].double())))
+    if kind in ("train", "logits"):
+        model = st["model"] if kind == "logits" else st["model"][0]
+        while hasattr(model, "module"):
+            model = model.module
+        names = [n for n, _ in model.named_parameters()]
+        w = {n: p.detach().double().requires_grad_(kind == "train") for n, p in model.named_parameters()}
+        if kind == "logits":
+            with torch.no_grad():
+                return _logits(c, w, st["tokens"])
+        loss = 0.0
+        for b in st["batches"]:
+            part = torch.nn.functional.cross_entropy(_logits(c, w, b["tokens"].cuda()).flatten(0, 1), b["labels"].cuda().flatten()) / len(st["batches"])
+            part.backward()
+            loss += float(part.detach())
+        grads = [w[n].grad for n in names]
+        norm = float(torch.stack([g.square().sum() for g in grads]).sum().sqrt())
+        return {"loss": loss, "grad_norm": norm, "weights": [None] * len(names), "grads": grads}        # clipped inside the update
+    w = {n: p.detach().double().requires_grad_(True) for n, p in st["module"].named_parameters()}
+    x, dout = st["x"].detach().double().requires_grad_(True), st["dout"].double()
+    if kind == "moe":
+        out, balance = _experts(c, w, x)
+        balance.backward(retain_graph=True)
+    else:
+        out = _latent_attention(c, w, x) if kind == "mla" else x @ w["weight"].t()
+    out.backward(dout)
+    return {"out": out.detach(), "dx": x.grad, "grads": {n: p.grad for n, p in w.items()}}

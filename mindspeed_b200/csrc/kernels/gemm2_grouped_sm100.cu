@@ -5,9 +5,10 @@
 //             [N_out, K_red]): X is K-major, W comes from one 3-D tensor map over the stacked weights [E, ., .]
 //   GG_WGRAD  dW[e][Kx, N] (+)= X[rows of e, Kx]^T * dY[rows of e, N]   reduction over the expert's rows, both operands
 //             MN-major; output through a 3-D tensor map over the stacked [E, Kx, N] tensor: bf16 / fp32 store or fp32
-//             reduce-add (accumulation into main_grad).  Only whole 64-row blocks of every expert are reduced
-//             (rows [start_e, start_e + 64 * floor(n_e / 64))); the caller adds the remaining < 64 rows per expert with a
-//             second launch on zero-padded copies (mindspeed_b200/ops/grouped_gemm.py).
+//             reduce-add (accumulation into main_grad).  The last, partial 64-row block of an expert is read from a
+//             zero-padded copy that a small kernel makes first, so that no row of the next expert enters the sum and the
+//             fp32 gradients are read and written once.  (They were read and written twice while the partial blocks went
+//             through a second launch: at 384 - 1024 rows an expert that traffic is what bounds the pass.)
 //
 // Expert e owns rows [offs[e], offs[e+1]) (int32 prefix sums in global memory).  A tile is (expert, 256-row block of the
 // expert, 256-column block); tiles are numbered expert by expert and dealt round-robin to the CTA pairs; every role
@@ -36,6 +37,7 @@ enum Epi : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_F32_ACC = 2 };
 struct GroupedParams {
   CUtensorMap tmA;        // GG_ROWS: X [rows, K] box [128 x 64];  GG_WGRAD: X [rows, Kx] box [64 rows x 64]
   CUtensorMap tmB;        // GG_ROWS: W 3-D {inner, outer, E};     GG_WGRAD: dY [rows, N] box [64 rows x 64]
+  CUtensorMap tmAt, tmBt; // GG_WGRAD: the zero-padded copies of the partial blocks, X [64 E, Kx] and dY [64 E, N]
   CUtensorMap tmD;        // GG_ROWS: Y [rows, N] box [32 x 64];   GG_WGRAD: dW 3-D {N, Kx, E} box [64|32, 32, 1]
   const int* offs;        // [E + 1] row prefix sums
   void* D;                // GG_ROWS: Y base for the predicated edge stores
@@ -89,7 +91,7 @@ struct TileCursor {
         t(pair), stride(npairs) {}
   __device__ int tiles_of(int s, int en) const {
     if (MODE == GG_ROWS) return ((en - s + 2 * BM - 1) / (2 * BM)) * num_n;
-    return (en - s) >= BK ? kx_tiles * num_n : 0;       // no whole 64-row block: nothing to reduce here
+    return en > s ? kx_tiles * num_n : 0;               // an expert without rows adds nothing
   }
   // false when the sequence is exhausted
   __device__ bool next(int& m_blk, int& n_blk) {
@@ -151,7 +153,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) gemm2_groupe
         const int n0 = n_blk * BN + (int)cta * (BN / 2);
         int num_kb, m0;
         if (MODE == GG_ROWS) { num_kb = (p.K + BK - 1) / BK; m0 = cur.start + m_blk * (2 * BM) + (int)cta * BM; }
-        else { num_kb = (cur.end - cur.start) / BK; m0 = m_blk * (2 * BM) + (int)cta * BM; }
+        else { num_kb = (cur.end - cur.start + BK - 1) / BK; m0 = m_blk * (2 * BM) + (int)cta * BM; }
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, p.status, 0x10u)) { alive = false; break; }
           const uint32_t sa = smem_base + stage * L::STAGE_BYTES;
@@ -169,11 +171,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) gemm2_groupe
                 tma_load_3d_pair(sb + j * (BK * 128), &p.tmB, lead_full, n0 + j * 64, k0, cur.e);
             }
           } else {
-            const int r0 = cur.start + kb * BK;                                                 // 64 rows of the expert
+            const bool part = cur.start + kb * BK + BK > cur.end;
+            const CUtensorMap *ta = part ? &p.tmAt : &p.tmA, *tb = part ? &p.tmBt : &p.tmB;
+            const int r0 = part ? cur.e * BK : cur.start + kb * BK;                             // 64 rows of the expert
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * (BK * 128), &p.tmA, lead_full, m0 + j * 64, r0);
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * (BK * 128), ta, lead_full, m0 + j * 64, r0);
 #pragma unroll
-            for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * (BK * 128), &p.tmB, lead_full, n0 + j * 64, r0);
+            for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sb + j * (BK * 128), tb, lead_full, n0 + j * 64, r0);
           }
           if (++stage == NSTAGE) { stage = 0; phase ^= 1u; }
         }
@@ -193,7 +197,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) gemm2_groupe
       TileCursor<MODE> cur(p, pair, npairs);
       int m_blk, n_blk;
       while (alive && cur.next(m_blk, n_blk)) {
-        const int num_kb = (MODE == GG_ROWS) ? (p.K + BK - 1) / BK : (cur.end - cur.start) / BK;
+        const int num_kb = ((MODE == GG_ROWS ? p.K : cur.end - cur.start) + BK - 1) / BK;
         if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, p.status, 0x20u)) { alive = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
@@ -329,6 +333,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) gemm2_groupe
   }
 }
 
+// Copies the partial last 64-row block of every expert into rows 64 e .. 64 e + 63 of xt [64 E, Kx] and yt [64 E, N] and fills it up
+// with zeros; blocks of experts without one are not read by the GEMM and stay as they are.
+__global__ void wgrad_tails_kernel(const uint4* __restrict__ x, const uint4* __restrict__ y, uint4* __restrict__ xt, uint4* __restrict__ yt,
+                                   const int* __restrict__ offs, int kv, int nv) {
+  const int e = (int)blockIdx.x >> 6, r = (int)blockIdx.x & 63;
+  const int start = offs[e], end = offs[e + 1], tail = (end - start) & (BK - 1);
+  if (tail == 0) return;
+  const size_t src = (size_t)(end - tail + r), dst = blockIdx.x;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int c = threadIdx.x; c < kv + nv; c += blockDim.x) {
+    if (c < kv) xt[dst * kv + c] = r < tail ? x[src * kv + c] : zero;
+    else yt[dst * nv + (c - kv)] = r < tail ? y[src * nv + (c - kv)] : zero;
+  }
+}
+
 template <int NSTAGE, int MODE, int EPI, bool B_MN>
 int launch_grouped(const GroupedParams& p, int pairs, cudaStream_t s) {
   using L = SmemG<NSTAGE, EPI>;
@@ -375,10 +394,10 @@ MSB_API int msb_grouped_gemm_rows(const void* X, const void* W, void* Y, const i
   return w_is_kn ? launch_grouped<6, GG_ROWS, EPI_BF16, true>(p, pairs, s) : launch_grouped<6, GG_ROWS, EPI_BF16, false>(p, pairs, s);
 }
 
-// dW[e][Kx, N] (+)= X[rows of e, Kx]^T * dY[rows of e, N] over the whole 64-row blocks of every expert.
-//   epilogue 0: bf16 store, 1: fp32 store, 2: fp32 accumulate.  Experts with fewer than 64 rows are not written at all.
-MSB_API int msb_grouped_gemm_wgrad(const void* X, const void* dY, void* dW, const int* offs, int E, int rows_total, int Kx, int N,
-                                   int epilogue, unsigned int* status, cudaStream_t s) {
+// dW[e][Kx, N] (+)= X[rows of e, Kx]^T * dY[rows of e, N].  x_tails [64 E, Kx] and dy_tails [64 E, N]: bf16 scratch.
+//   epilogue 0: bf16 store, 1: fp32 store, 2: fp32 accumulate.  Experts without rows are not written at all.
+MSB_API int msb_grouped_gemm_wgrad(const void* X, const void* dY, void* dW, const int* offs, void* x_tails, void* dy_tails, int E,
+                                   int rows_total, int Kx, int N, int epilogue, unsigned int* status, cudaStream_t s) {
   MSB_REQUIRE(E > 0 && rows_total > 0 && N % 8 == 0 && Kx % 8 == 0, "grouped_gemm_wgrad: bad shape E=%d rows=%d Kx=%d N=%d", E, rows_total, Kx, N);
   MSB_REQUIRE(status != nullptr, "grouped_gemm_wgrad: status word is required");
   GroupedParams p;
@@ -387,6 +406,12 @@ MSB_API int msb_grouped_gemm_wgrad(const void* X, const void* dY, void* dW, cons
   if (rc) return rc;
   rc = make_tmap_2d(&p.tmB, dY, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows_total, N, N, BK, 64);
   if (rc) return rc;
+  rc = make_tmap_2d(&p.tmAt, x_tails, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)E * BK, Kx, Kx, BK, 64);
+  if (rc) return rc;
+  rc = make_tmap_2d(&p.tmBt, dy_tails, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)E * BK, N, N, BK, 64);
+  if (rc) return rc;
+  wgrad_tails_kernel<<<E * BK, 256, 0, s>>>((const uint4*)X, (const uint4*)dY, (uint4*)x_tails, (uint4*)dy_tails, offs, Kx / 8, N / 8);
+  MSB_CHECK_LAUNCH("grouped_wgrad_tails");
   if (epilogue == EPI_BF16) rc = make_map3(&p.tmD, dW, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, Kx, E, 64, 32);
   else rc = make_map3(&p.tmD, dW, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, N, Kx, E, 32, 32);
   if (rc) return rc;

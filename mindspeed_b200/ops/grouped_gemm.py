@@ -3,8 +3,8 @@
 On a GPU forward, data gradient and weight gradient are each ONE launch of the CTA-pair grouped kernel
 (csrc/kernels/gemm2_grouped_sm100.cu) over all experts; the experts' row ranges travel as an int32 prefix-sum tensor on the
 device, so a ``tokens_per_expert`` tensor is never read back to the host.  The weight gradient accumulates straight into the
-fp32 ``main_grad`` of the stacked weight when present; its reduction runs over the whole 64-row blocks of every expert in
-the main launch and over a zero-padded copy of the remaining (< 64) rows per expert in a second, small launch.
+fp32 ``main_grad`` of the stacked weight when present; the last, partial 64-row block of every expert is read from a
+zero-padded copy.
 The CPU path is the eager loop and serves as the oracle.  reference semantics: npu_gmm / npu_gmm_backward
 (mindspeed/ops/gmm.py:20-175, mindspeed/ops/csrc/cann/gmm.cpp:169-300: dx = dy W^T, dw = x^T dy grouped on K).
 """
@@ -48,30 +48,15 @@ def _rows(x, w, y, offs, n_out, k_red, w_is_kn):
     return y
 
 
-def _wgrad(x, dy, dw, offs, epilogue):
-    L = loader.require_lib()
-    st = G.status_word(x.device)
-    loader.check(L.msb_grouped_gemm_wgrad(loader.p(x), loader.p(dy), loader.p(dw), loader.p(offs), dw.shape[0], x.shape[0], x.shape[1],
-                                          dy.shape[1], int(epilogue), loader.p(st), ctypes.c_void_p(loader.stream_ptr())),
-                 "grouped_gemm_wgrad")
-
-
 def grouped_wgrad_acc(x, dy, offs, acc):
     """acc[e] (fp32 [E, K, N]) += x[rows of e]^T @ dy[rows of e], rows given by the device prefix sums ``offs``."""
+    L = loader.require_lib()
     E = acc.shape[0]
-    _wgrad(x, dy, acc, offs, G.EPI_F32_ACC)                  # whole 64-row blocks of every expert
-    # the < 64 trailing rows of every expert, gathered into zero-padded [E, 64, .] copies (all on the device)
-    end = offs[1:].long()
-    n = end - offs[:-1].long()
-    tail = n % TAIL
-    r = torch.arange(TAIL, device=x.device).view(1, TAIL)
-    idx = (end - tail).view(E, 1) + r
-    valid = r < tail.view(E, 1)
-    idx = torch.where(valid, idx, torch.zeros_like(idx)).view(-1)
-    xt = x.index_select(0, idx) * valid.view(-1, 1).to(x.dtype)
-    dyt = dy.index_select(0, idx)
-    offs2 = torch.arange(E + 1, device=x.device, dtype=torch.int32) * TAIL
-    _wgrad(xt, dyt, acc, offs2, G.EPI_F32_ACC)
+    st = G.status_word(x.device)
+    xt, dyt = (torch.empty(E * TAIL, t.shape[1], dtype=t.dtype, device=t.device) for t in (x, dy))
+    loader.check(L.msb_grouped_gemm_wgrad(loader.p(x), loader.p(dy), loader.p(acc), loader.p(offs), loader.p(xt), loader.p(dyt), E,
+                                          x.shape[0], x.shape[1], dy.shape[1], int(G.EPI_F32_ACC), loader.p(st),
+                                          ctypes.c_void_p(loader.stream_ptr())), "grouped_gemm_wgrad")
 
 
 def grouped_gemm_ref(x, w, tokens_per_expert):

@@ -1,0 +1,51 @@
+"""Edges of the vectorised reduction, row-scale gradient and row scatter-add kernels."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 4099, 1 << 20, (1 << 24) + 5])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_l2norm_lengths_and_alignment(n, offset, dtype):
+    """Sums of squares (all positive) in fp32 over fewer than 2^10 terms a thread: relative error below 2^10 * 2^-24."""
+    from mindspeed_b200.ops import adam as A
+    torch.manual_seed(n)
+    g = torch.randn(n + offset, device="cuda").to(dtype)[offset:]
+    ref = g.double().square().sum().item()
+    assert abs(A.l2norm_sq(g).item() - ref) <= 6.2e-5 * ref
+
+
+@pytest.mark.parametrize("rows,F", [(1, 8), (3, 264), (5000, 64), (37, 14336)])
+def test_swiglu_row_scale_gradient(rows, F):
+    """bf16 inputs, fp32 sums of F products: the oracle is the same expression in 64 bits; outputs round to bf16."""
+    from mindspeed_b200.ops.activation import swiglu
+    torch.manual_seed(F)
+    x = torch.randn(rows, 2 * F, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    sc = torch.rand(rows, device="cuda", requires_grad=True)
+    dy = torch.randn(rows, F, device="cuda", dtype=torch.bfloat16)
+    swiglu(x, sc).backward(dy)
+    xd, sd = x.detach().double().requires_grad_(True), sc.detach().double().requires_grad_(True)
+    a, b = xd.chunk(2, -1)
+    (torch.nn.functional.silu(a) * b * sd[:, None]).backward(dy.double())
+    assert ((sc.grad - sd.grad).norm() / sd.grad.norm()).item() < 1e-5
+    assert ((x.grad - xd.grad).norm() / xd.grad.norm()).item() < 4e-3
+
+
+@pytest.mark.parametrize("n,rows,cols", [(1, 1, 8), (7, 3, 24), (300, 40, 1000), (6 * 128, 128, 4096), (500, 2, 2048), (64, 1, 133), (65, 1, 136)])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_scatter_add_rows(n, rows, cols, weighted, dtype):
+    """Repeated and missing targets, more than one list of 64, columns that no vector divides; fp32 sums, one rounding."""
+    from mindspeed_b200.ops.permute import scatter_add_rows
+    torch.manual_seed(n + cols)
+    src = torch.randn(n, cols, device="cuda").to(dtype)
+    idx = torch.randint(0, max(1, rows - 1), (n,), device="cuda")
+    w = torch.rand(n, device="cuda") if weighted else None
+    want = torch.zeros(rows, cols, device="cuda", dtype=torch.float64)
+    want.index_add_(0, idx, src.double() * (1.0 if w is None else w.double()[:, None]))
+    got = scatter_add_rows(src, idx, rows, w)
+    assert got.dtype == dtype
+    tol = 4e-3 if dtype == torch.bfloat16 else 3e-5
+    assert ((got.double() - want).abs() <= tol * want.abs() + 3e-5 * want.abs().max()).all()

@@ -267,6 +267,11 @@ class MLASelfAttention(nn.Module):
             kv_in = M.scatter_to_sequence_parallel_region(kv_lat) if sp else kv_lat
             kv = up(self.linear_kv_up_proj, kv_in)
             kv = kv.view(s, b, self.n, self.qk_nope + self.v_dim)
+        if not self.dsa and rotary_pos_emb is not None and cfg.optimization_level >= 1:
+            from ..ops.mla_heads import mla_heads
+            qf, kf, v = mla_heads(q, kv, k_pe, *rotary_pos_emb, self.qk_nope, cfg.rotary_interleaved)
+            return self._attend(qf, kf, v, attention_mask, packed_seq_params)
+        if not self.dsa:
             k_nope, v = kv.split([self.qk_nope, self.v_dim], dim=-1)
         q_nope, q_pe = q.split([self.qk_nope, self.qk_rope], dim=-1)
         k_pe = k_pe.reshape(s, b, 1, self.qk_rope)
@@ -284,14 +289,17 @@ class MLASelfAttention(nn.Module):
             ctx = dsa_attention(self, xf, qcf, qf, kv_lat, k_pe, rotary_pos_emb)
             return self.linear_proj(ctx)
         kf = torch.cat((k_nope, k_pe.expand(s, b, self.n, self.qk_rope)), dim=-1)
-        if getattr(cfg, "mla_swap_core_attn_out", False) and self.training and torch.is_grad_enabled() and qf.is_cuda:
+        return self._attend(qf, kf, v.contiguous(), attention_mask, packed_seq_params)
+
+    def _attend(self, qf, kf, v, attention_mask, packed_seq_params):
+        if getattr(self.config, "mla_swap_core_attn_out", False) and self.training and torch.is_grad_enabled() and qf.is_cuda:
             # --mla-swap-core-attn-out: what the attention keeps for backward (q, k, v, output, softmax statistics) waits in
             # pinned host memory
             from ..memory.host_offload import OffloadSaved
             with OffloadSaved():
-                ctx = self.core_attention(qf, kf, v.contiguous(), attention_mask, packed_seq_params)
+                ctx = self.core_attention(qf, kf, v, attention_mask, packed_seq_params)
         else:
-            ctx = self.core_attention(qf, kf, v.contiguous(), attention_mask, packed_seq_params)
+            ctx = self.core_attention(qf, kf, v, attention_mask, packed_seq_params)
         return self.linear_proj(ctx)
 
 

@@ -31,7 +31,8 @@ constexpr float RESCALE_THRESHOLD = 8.f;  // log2 units
 constexpr int P_HEAD = 96;                // keys of a tile whose probabilities are handed to the MMA first
 
 struct Fwd2Params {
-  CUtensorMap tmQ, tmK, tmV, tmO;  // dims {d, head, batch, seq}
+  CUtensorMap tmQ;                 // dims {d, head of the group, group, batch, seq}: the heads of a packed QKV activation are not evenly spaced
+  CUtensorMap tmK, tmV, tmO;       // dims {d, head, batch, seq}
   float* lse;                      // [b, nq, sq]
   __nv_bfloat16* O;                // [sq, b, nq, d] (direct stores for rows without any visible key)
   int sq, sk, b, nq, nkv;
@@ -51,6 +52,12 @@ struct Fwd2Smem {
 
 __device__ __forceinline__ void named_bar(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* tmap, uint32_t bar, int x, int y, int z, int v, int w) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(v), "r"(w)
+      : "memory");
+}
 __device__ __forceinline__ void tma_store_4d(const void* tmap, uint32_t src, int x, int y, int z, int w) {
   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(tmap)),
@@ -127,8 +134,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const uint32_t qs = base + Fwd2Smem::Q_OFF + t * TILE_BYTES;
-        tma_load_4d(qs, &p.tmQ, q_full, 0, head, batch, q0 + t * FB);
-        tma_load_4d(qs + HALF_BYTES, &p.tmQ, q_full, 64, head, batch, q0 + t * FB);
+        tma_load_5d(qs, &p.tmQ, q_full, 0, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
+        tma_load_5d(qs + HALF_BYTES, &p.tmQ, q_full, 64, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
       }
       bool ok = true;
       for (int j = 0; j < n_max && ok; ++j) {
@@ -353,19 +360,27 @@ int make_map4(CUtensorMap* tm, const void* base, int seq, int heads, int b, long
   uint32_t box[4] = {64, 1, 1, (uint32_t)FB};
   return make_tmap_nd(tm, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 4, dims, str, box);
 }
+// queries: groups of `rep` heads, strides between heads of a group (sh) and between groups (gs)
+int make_map_q(CUtensorMap* tm, const void* base, int seq, int rep, int groups, int b, long long ss, long long sb, long long gs, long long sh) {
+  uint64_t dims[5] = {(uint64_t)FD, (uint64_t)rep, (uint64_t)groups, (uint64_t)b, (uint64_t)seq};
+  uint64_t str[4] = {(uint64_t)sh * 2, (uint64_t)gs * 2, (uint64_t)sb * 2, (uint64_t)ss * 2};
+  uint32_t box[5] = {64, 1, 1, 1, (uint32_t)FB};
+  return make_tmap_nd(tm, base, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 5, dims, str, box);
+}
 }  // namespace
 
-// q [sq, b, nq, 128], k / v [sk, b, nkv, 128] bf16 with element strides (seq, batch, head), last dim contiguous;
+// q [sq, b, nkv, nq / nkv, 128] with element strides (seq, batch, group, head), k / v [sk, b, nkv, 128] with (seq, batch, head), bf16, last
+// dim contiguous;
 // o [sq, b, nq, 128] contiguous; lse [b, nq, sq] fp32 (natural log of the scaled scores' softmax denominator).
 MSB_API int msb_flash_fwd2(const void* q, const void* k, const void* v, void* o, float* lse, int sq, int sk, int b, int nq, int nkv,
-                           long long q_ss, long long q_sb, long long q_sh, long long k_ss, long long k_sb, long long k_sh,
+                           long long q_ss, long long q_sb, long long q_gs, long long q_sh, long long k_ss, long long k_sb, long long k_sh,
                            long long v_ss, long long v_sb, long long v_sh, int causal, int q_offset, float scale,
                            unsigned int* status, cudaStream_t s) {
   MSB_REQUIRE(sq > 0 && sk > 0 && nq % nkv == 0, "flash_fwd2: bad shape sq=%d sk=%d nq=%d nkv=%d", sq, sk, nq, nkv);
   MSB_REQUIRE(status != nullptr, "flash_fwd2: status word is required");
   Fwd2Params p;
   memset(&p, 0, sizeof(p));
-  int rc = make_map4(&p.tmQ, q, sq, nq, b, q_ss, q_sb, q_sh); if (rc) return rc;
+  int rc = make_map_q(&p.tmQ, q, sq, nq / nkv, nkv, b, q_ss, q_sb, q_gs, q_sh); if (rc) return rc;
   rc = make_map4(&p.tmK, k, sk, nkv, b, k_ss, k_sb, k_sh); if (rc) return rc;
   rc = make_map4(&p.tmV, v, sk, nkv, b, v_ss, v_sb, v_sh); if (rc) return rc;
   rc = make_map4(&p.tmO, o, sq, nq, b, (long long)b * nq * FD, (long long)nq * FD, FD); if (rc) return rc;
@@ -414,7 +429,8 @@ MSB_API int msb_flash_fwd2(const void* q, const void* k, const void* v, void* o,
 namespace {
 
 struct BwdParams {
-  CUtensorMap tmQ, tmK, tmV, tmdO;  // bf16, dims {d, head, batch, seq}
+  CUtensorMap tmQ;                  // bf16, dims {d, head of the group, group, batch, seq}
+  CUtensorMap tmK, tmV, tmdO;       // bf16, dims {d, head, batch, seq}
   CUtensorMap tmdQ;                 // fp32 [sq, b, nq, d], dims {d, head, batch, seq}, box {32, 1, 1, 32}
   CUtensorMap tmdK, tmdV;           // [sk, b, nkv, d] outputs: bf16 stores, or fp32 reduce-add targets (box {32,1,1,32}) when split_heads
   const float* nlse2;               // [b, nq, sq_pad] -LSE * log2(e) (-inf where no key is visible / padding)
@@ -452,33 +468,69 @@ __device__ __forceinline__ void tma_reduce_add_4d(const void* tmap, uint32_t src
                : "memory");
 }
 
-// delta[b, h, r] = sum_d dO * O; lse2 = LSE * log2(e) with -inf (no visible key) and padding rows mapped to +inf.
-__global__ void flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, long long do_ss,
-                                      long long do_sb, long long do_sh, const float* __restrict__ lse, float* __restrict__ nlse2,
-                                      float* __restrict__ ndelta, int sq, int b, int nq, int sq_pad) {
-  const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  const long long total = (long long)b * nq * sq_pad;
-  if (warp >= total) return;
-  const int r = warp % sq_pad, h = (warp / sq_pad) % nq, bb = warp / (sq_pad * nq);
-  float acc = 0.f, l2 = -INFINITY;
-  if (r < sq) {
-    const __nv_bfloat16* orow = o + (((size_t)r * b + bb) * nq + h) * FD + lane * 4;
-    const __nv_bfloat16* drow = dout + (size_t)r * do_ss + (size_t)bb * do_sb + (size_t)h * do_sh + lane * 4;
-    const uint2 ov = *reinterpret_cast<const uint2*>(orow), dv = *reinterpret_cast<const uint2*>(drow);
-    const __nv_bfloat162* oh = reinterpret_cast<const __nv_bfloat162*>(&ov);
-    const __nv_bfloat162* dh = reinterpret_cast<const __nv_bfloat162*>(&dv);
+// Statistics of the backward: ndelta[b, h, r] = -sum_d dO * O; nlse2 = -LSE * log2(e), with -inf for rows without a visible key and for the
+// padding to whole tiles.  Also clears the fp32 accumulators that the main kernel adds into (`zero4` vectors of four).  Bound by the
+// read of O and dO and the write of the zeros: 16 lanes per row, 16 bytes a lane.
+__global__ void __launch_bounds__(256) flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, long long do_ss,
+                                                             long long do_sb, long long do_sh, const float* __restrict__ lse,
+                                                             float* __restrict__ nlse2, float* __restrict__ ndelta, int sq, int b, int nq, int sq_pad,
+                                                             float4* __restrict__ zero, long long zero4) {
+  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;
+  for (long long i = tid; i < zero4; i += threads) zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int l16 = threadIdx.x & 15;
+  // row numbers run with the sequence slowest, as O and dO lie in memory; every lane of a warp makes the same number of rounds
+  const long long total = (long long)sq_pad * b * nq;
+  for (long long w0 = (tid >> 5) * 2; w0 < total; w0 += (threads >> 5) * 2) {
+    const long long w = w0 + ((threadIdx.x >> 4) & 1);
+    const int h = (int)(w % nq), bb = (int)((w / nq) % b);
+    const long long row = w / ((long long)nq * b);
+    const bool live = w < total && row < sq;
+    float acc = 0.f;
+    if (live) {
+      const uint4 ov = *reinterpret_cast<const uint4*>(o + w * FD + l16 * 8);
+      const uint4 dv = *reinterpret_cast<const uint4*>(dout + row * do_ss + bb * do_sb + h * do_sh + l16 * 8);
+      const __nv_bfloat162* oh = reinterpret_cast<const __nv_bfloat162*>(&ov);
+      const __nv_bfloat162* dh = reinterpret_cast<const __nv_bfloat162*>(&dv);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float2 a = __bfloat1622float2(oh[i]), c = __bfloat1622float2(dh[i]);
-      acc += a.x * c.x + a.y * c.y;
+      for (int i = 0; i < 4; ++i) {
+        const float2 a = __bfloat1622float2(oh[i]), c = __bfloat1622float2(dh[i]);
+        acc += a.x * c.x + a.y * c.y;
+      }
     }
-    acc = warp_sum(acc);
-    const float l = lse[((size_t)bb * nq + h) * sq + r];
-    l2 = (l == -INFINITY) ? -INFINITY : l * -1.4426950408889634f;
+#pragma unroll
+    for (int d = 8; d; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (l16 == 0 && w < total) {
+      const float l = live ? lse[((size_t)bb * nq + h) * sq + row] : -INFINITY;
+      const size_t at = ((size_t)bb * nq + h) * sq_pad + row;
+      ndelta[at] = -acc;
+      nlse2[at] = (l == -INFINITY) ? -INFINITY : l * -1.4426950408889634f;
+    }
   }
-  if (lane == 0) {
-    ndelta[warp] = -acc;
-    nlse2[warp] = l2;
+}
+
+// fp32 sums -> bf16 gradients at their place: dQ always, dK and dV when query heads added into fp32 buffers.  16 lanes per 128-wide row.
+struct FinishSeg {
+  const float* src;                 // [rows, 128]
+  __nv_bfloat16* dst;
+  long long ss, sb, gs, sh;         // element strides of dst
+  int b, groups, per;               // row = ((seq * b + batch) * groups + group) * per + head of the group
+  long long rows;
+};
+struct FinishParams { FinishSeg seg[3]; };
+__global__ void __launch_bounds__(256) flash_bwd_finish_kernel(const __grid_constant__ FinishParams p) {
+  const int l16 = threadIdx.x & 15;
+  const long long r1 = p.seg[0].rows, r2 = r1 + p.seg[1].rows, all = r2 + p.seg[2].rows;
+  for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 4; r < all; r += ((long long)gridDim.x * blockDim.x) >> 4) {
+    const FinishSeg& g = p.seg[r < r1 ? 0 : r < r2 ? 1 : 2];
+    const long long w = r - (r < r1 ? 0 : r < r2 ? r1 : r2);
+    const float4* src = reinterpret_cast<const float4*>(g.src + w * FD) + 2 * l16;
+    const float4 x = src[0], y = src[1];
+    const int h = (int)(w % g.per);
+    long long t = w / g.per;
+    const int gr = (int)(t % g.groups);
+    t /= g.groups;
+    __nv_bfloat16* dst = g.dst + (t / g.b) * g.ss + (t % g.b) * g.sb + gr * g.gs + h * g.sh + l16 * 8;
+    *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w), pack_bf16(y.x, y.y), pack_bf16(y.z, y.w));
   }
 }
 
@@ -503,11 +555,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // key tiles that many query tiles see (early ones, when causal) first, over all heads: the last CTAs to start are the shortest
-  const int j = (int)blockIdx.y;
+  const int heads = p.split_heads ? p.nq : p.nkv, head_id = (int)(blockIdx.x % (unsigned)heads), j = (int)(blockIdx.x / (unsigned)heads);
   // without the split a CTA walks all query heads of its KV head; with it (few KV heads: too few CTAs otherwise) one each
   const int rep_all = p.nq / p.nkv;
-  const int g = p.split_heads ? (int)blockIdx.x / rep_all : (int)blockIdx.x, batch = blockIdx.z;
-  const int head0 = p.split_heads ? (int)blockIdx.x : g * rep_all;
+  const int g = p.split_heads ? head_id / rep_all : head_id, batch = blockIdx.z;
+  const int head0 = p.split_heads ? head_id : g * rep_all;
   const int rep = p.split_heads ? 1 : rep_all;
   const int key0 = j * FB;
   const int n_q = (p.sq + FB - 1) / FB;
@@ -550,8 +602,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
         mbar_arrive_expect_tx(q_full(s), TILE_BYTES + BwdSmem::STAT_BYTES);
         const uint32_t qs = base + BwdSmem::Q_OFF + s * TILE_BYTES, ss = base + BwdSmem::STAT_OFF + s * BwdSmem::STAT_BYTES;
         const size_t stat = ((size_t)batch * p.nq + head) * p.sq_pad + (size_t)i * FB;
-        tma_load_4d(qs, &p.tmQ, q_full(s), 0, head, batch, i * FB);
-        tma_load_4d(qs + HALF_BYTES, &p.tmQ, q_full(s), 64, head, batch, i * FB);
+        tma_load_5d(qs, &p.tmQ, q_full(s), 0, head - g * rep_all, g, batch, i * FB);
+        tma_load_5d(qs + HALF_BYTES, &p.tmQ, q_full(s), 64, head - g * rep_all, g, batch, i * FB);
         bulk_g2s_bar(ss, p.nlse2 + stat, FB * 4, q_full(s));
         bulk_g2s_bar(ss + FB * 4, p.ndelta + stat, FB * 4, q_full(s));
         if (!mbar_wait(do_empty, (uint32_t)(it & 1) ^ 1u, p.status, 0x411u)) break;
@@ -752,7 +804,23 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
       if (lane == 0) tma_store_wait<0>();
     }
     // ---- dK, dV of this key tile: TMEM -> bf16 -> shared memory (the Q stage buffers) -> TMA store; compute warps only ----
-    if (n_it > 0 && ch < 2) {
+    if (n_it == 0) {
+      // no query sees this tile: its gradients are zero (with the split the fp32 buffers are)
+      if (!p.split_heads && ch < 2) {
+        uint4* z = reinterpret_cast<uint4*>(base_ptr + BwdSmem::Q_OFF);
+        for (int c = (int)threadIdx.x - 64; c < TILE_BYTES / 16; c += 256) z[c] = make_uint4(0, 0, 0, 0);
+        fence_proxy_async_smem();
+        named_bar(2, 256);
+        if (warp == 2 && lane == 0) {
+          for (int x = 0; x < 2; ++x) {
+            tma_store_4d(&p.tmdV, base + BwdSmem::Q_OFF, 64 * x, g, batch, key0);
+            tma_store_4d(&p.tmdK, base + BwdSmem::Q_OFF, 64 * x, g, batch, key0);
+          }
+          tma_store_commit();
+          tma_store_wait<0>();
+        }
+      }
+    } else if (ch < 2) {
       if (ok) ok = mbar_wait(acc_done, 0, p.status, 0x434u);
       tc_fence_after();
       if (p.split_heads) {
@@ -828,52 +896,52 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
 }
 }  // namespace
 
-// Gradients of flash attention.  q / k / v / dout strided like the forward's inputs, o [sq, b, nq, 128] contiguous,
-// lse [b, nq, sq]; dq32 [sq, b, nq, 128] fp32 ZERO-INITIALISED by the caller (key tiles add into it), dk / dv
-// [sk, b, nkv, 128] bf16 contiguous, zero-initialised when some key tile is visible to no query; nlse2 / ndelta: scratch
-// fp32 [b, nq, ceil(sq / 128) * 128] each.
-// split_heads = 1: dk / dv are fp32 [sk, b, nkv, 128] ZERO-INITIALISED buffers that every query head adds into (use when
-// ceil(sk / 128) * nkv * b is well below the SM count); 0: bf16 outputs written once.
-MSB_API int msb_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
-                          float* dq32, void* dk, void* dv, float* nlse2, float* ndelta, int split_heads, int sq, int sk, int b, int nq, int nkv,
-                          long long q_ss, long long q_sb, long long q_sh, long long k_ss, long long k_sb, long long k_sh,
+// Gradients of flash attention.  q / k / v strided like the forward's inputs, dout [sq, b, nq, 128] with strides (seq, batch, head), o
+// [sq, b, nq, 128] contiguous, lse [b, nq, sq].  dq / dk / dv: bf16, strides as q / k / v, last dim contiguous, every row written.
+// acc: fp32 scratch, sq * b * nq * 128 elements for dQ, and with split_heads 2 * sk * b * nkv * 128 more for dK and dV; nlse2 / ndelta:
+// fp32 scratch [b, nq, ceil(sq / 128) * 128] each.  All 16-byte aligned.
+// split_heads = 1: one CTA per query head, which add their dK / dV in fp32 (use when ceil(sk / 128) * nkv * b is well below twice the SM
+// count); 0: one CTA per KV head, dK / dV written once.
+MSB_API int msb_flash_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse, float* acc,
+                          void* dq, void* dk, void* dv, float* nlse2, float* ndelta, int split_heads, int sq, int sk, int b, int nq, int nkv,
+                          long long q_ss, long long q_sb, long long q_gs, long long q_sh, long long k_ss, long long k_sb, long long k_sh,
                           long long v_ss, long long v_sb, long long v_sh, long long do_ss, long long do_sb, long long do_sh,
-                          int causal, int q_offset, float scale, unsigned int* status, cudaStream_t s) {
+                          long long dq_ss, long long dq_sb, long long dq_gs, long long dq_sh, long long dk_ss, long long dk_sb, long long dk_sh,
+                          long long dv_ss, long long dv_sb, long long dv_sh, int causal, int q_offset, float scale, unsigned int* status,
+                          cudaStream_t s) {
   MSB_REQUIRE(sq > 0 && sk > 0 && nq % nkv == 0, "flash_bwd: bad shape sq=%d sk=%d nq=%d nkv=%d", sq, sk, nq, nkv);
   MSB_REQUIRE(status != nullptr, "flash_bwd: status word is required");
   const int sq_pad = (sq + FB - 1) / FB * FB;
+  const long long q_rows = (long long)sq * b * nq, k_rows = (long long)sk * b * nkv;
+  float *dk32 = acc + q_rows * FD, *dv32 = dk32 + k_rows * FD;
   {
-    const long long rows = (long long)b * nq * sq_pad;
-    const int threads = 256;
-    const long long blocks = (rows * 32 + threads - 1) / threads;
-    flash_bwd_prep_kernel<<<(unsigned)blocks, threads, 0, s>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, do_ss, do_sb, do_sh,
-                                                             lse, nlse2, ndelta, sq, b, nq, sq_pad);
+    const long long pairs = ((long long)b * nq * sq_pad + 1) / 2, blocks = (pairs + 7) / 8, most = (long long)msb::num_sms() * 32;
+    flash_bwd_prep_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, s>>>(
+        (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, do_ss, do_sb, do_sh, lse, nlse2, ndelta, sq, b, nq, sq_pad, (float4*)acc,
+        (q_rows + (split_heads ? 2 * k_rows : 0)) * (FD / 4));
     MSB_CHECK_LAUNCH("flash_bwd_prep");
   }
   BwdParams p;
   memset(&p, 0, sizeof(p));
-  int rc = make_map4(&p.tmQ, q, sq, nq, b, q_ss, q_sb, q_sh); if (rc) return rc;
+  int rc = make_map_q(&p.tmQ, q, sq, nq / nkv, nkv, b, q_ss, q_sb, q_gs, q_sh); if (rc) return rc;
   rc = make_map4(&p.tmK, k, sk, nkv, b, k_ss, k_sb, k_sh); if (rc) return rc;
   rc = make_map4(&p.tmV, v, sk, nkv, b, v_ss, v_sb, v_sh); if (rc) return rc;
   rc = make_map4(&p.tmdO, dout, sq, nq, b, do_ss, do_sb, do_sh); if (rc) return rc;
+  auto map32 = [&](CUtensorMap* tm, float* base, int seq, int heads) {       // contiguous fp32, boxes of 32 rows x 32 columns
+    uint64_t dims[4] = {(uint64_t)FD, (uint64_t)heads, (uint64_t)b, (uint64_t)seq};
+    uint64_t str[3] = {(uint64_t)FD * 4, (uint64_t)heads * FD * 4, (uint64_t)b * heads * FD * 4};
+    uint32_t box[4] = {32, 1, 1, 32};
+    return make_tmap_nd(tm, base, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 4, dims, str, box);
+  };
   if (!split_heads) {
-    rc = make_map4(&p.tmdK, dk, sk, nkv, b, (long long)b * nkv * FD, (long long)nkv * FD, FD); if (rc) return rc;
-    rc = make_map4(&p.tmdV, dv, sk, nkv, b, (long long)b * nkv * FD, (long long)nkv * FD, FD); if (rc) return rc;
+    rc = make_map4(&p.tmdK, dk, sk, nkv, b, dk_ss, dk_sb, dk_sh); if (rc) return rc;
+    rc = make_map4(&p.tmdV, dv, sk, nkv, b, dv_ss, dv_sb, dv_sh); if (rc) return rc;
   } else {
-    uint64_t dims[4] = {(uint64_t)FD, (uint64_t)nkv, (uint64_t)b, (uint64_t)sk};
-    uint64_t str[3] = {(uint64_t)FD * 4, (uint64_t)nkv * FD * 4, (uint64_t)b * nkv * FD * 4};
-    uint32_t box[4] = {32, 1, 1, 32};
-    rc = make_tmap_nd(&p.tmdK, dk, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 4, dims, str, box); if (rc) return rc;
-    rc = make_tmap_nd(&p.tmdV, dv, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 4, dims, str, box); if (rc) return rc;
+    rc = map32(&p.tmdK, dk32, sk, nkv); if (rc) return rc;
+    rc = map32(&p.tmdV, dv32, sk, nkv); if (rc) return rc;
   }
+  rc = map32(&p.tmdQ, acc, sq, nq); if (rc) return rc;
   p.split_heads = split_heads ? 1 : 0;
-  {
-    uint64_t dims[4] = {(uint64_t)FD, (uint64_t)nq, (uint64_t)b, (uint64_t)sq};
-    uint64_t str[3] = {(uint64_t)FD * 4, (uint64_t)nq * FD * 4, (uint64_t)b * nq * FD * 4};
-    uint32_t box[4] = {32, 1, 1, 32};
-    rc = make_tmap_nd(&p.tmdQ, dq32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 4, dims, str, box);
-    if (rc) return rc;
-  }
   p.nlse2 = nlse2; p.ndelta = ndelta;
   p.sq = sq; p.sk = sk; p.b = b; p.nq = nq; p.nkv = nkv; p.sq_pad = sq_pad; p.causal = causal; p.q_offset = q_offset;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
@@ -883,8 +951,18 @@ MSB_API int msb_flash_bwd(const void* q, const void* k, const void* v, const voi
     if (e != cudaSuccess) { msb_set_error("flash_bwd: cannot set dynamic shared memory: %s", cudaGetErrorString(e)); return 1; }
     attr = true;
   }
-  dim3 grid(split_heads ? nq : nkv, (sk + FB - 1) / FB, b);
+  const long long ctas = (long long)(split_heads ? nq : nkv) * ((sk + FB - 1) / FB);
+  MSB_REQUIRE(ctas <= 0x7fffffffll, "flash_bwd: grid too large (%lld)", ctas);
+  dim3 grid((unsigned)ctas, 1, b);
   flash_bwd_sm100_kernel<<<grid, BWD_THREADS, BwdSmem::TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("flash_bwd_sm100");
+  FinishParams fp;
+  FinishSeg* sg = fp.seg;
+  sg[0] = FinishSeg{acc, (__nv_bfloat16*)dq, dq_ss, dq_sb, dq_gs, dq_sh, b, nkv, nq / nkv, q_rows};
+  sg[1] = FinishSeg{dk32, (__nv_bfloat16*)dk, dk_ss, dk_sb, dk_sh, 0, b, nkv, 1, split_heads ? k_rows : 0};
+  sg[2] = FinishSeg{dv32, (__nv_bfloat16*)dv, dv_ss, dv_sb, dv_sh, 0, b, nkv, 1, split_heads ? k_rows : 0};
+  const long long fin = (sg[0].rows + sg[1].rows + sg[2].rows + 15) / 16, most = (long long)msb::num_sms() * 16;
+  flash_bwd_finish_kernel<<<(unsigned)(fin < most ? fin : most), 256, 0, s>>>(fp);
+  MSB_CHECK_LAUNCH("flash_bwd_finish");
   return 0;
 }

@@ -120,11 +120,31 @@ class CoreAttention(nn.Module):
             elif self.config.optimization_level >= 1 and want in ("auto", "sm100"):
                 backend = "sm100"
             out = attn_ops.flash_attention(q, k, v, causal=self.causal, softmax_scale=self.softmax_scale, backend=backend)
+        return self._finish(out)
+
+    def _finish(self, out):
         if self.dropout_p > 0 and self.training:
             with get_cuda_rng_tracker().fork():
                 out = torch.nn.functional.dropout(out, self.dropout_p)
         s, b = out.shape[0], out.shape[1]
         return out.reshape(s, b, -1)
+
+    def packed(self, qkv, rotary_pos_emb, groups, qpg, attention_mask, packed_seq_params):
+        """The attention of a packed QKV activation without taking it apart, or None where ``forward`` would not run the plain
+        self-attention of the hand-written kernels (or where somebody has hooked or replaced it)."""
+        cfg = self.config
+        if (type(self) is not CoreAttention or "forward" in self.__dict__ or self._forward_hooks or self._forward_pre_hooks
+                or self._backward_hooks or self._backward_pre_hooks):
+            return None
+        if (cfg.optimization_level < 1 or getattr(cfg, "attention_backend", "auto") not in ("auto", "sm100") or self.alibi_slopes is not None
+                or packed_seq_params is not None or (attention_mask is not None and not self.causal)
+                or ps.get_context_parallel_world_size() > 1 or self._window(qkv.shape[0], qkv.shape[0]) is not None or not qkv.is_cuda):
+            return None
+        from ..ops.flash_sm100_impl import flash_attention_packed, packed_supports
+        if not packed_supports(qkv, groups, qpg):
+            return None
+        cos, sin = rotary_pos_emb if rotary_pos_emb is not None else (None, None)
+        return self._finish(flash_attention_packed(qkv, cos, sin, groups, qpg, cfg.rotary_interleaved, self.causal, self.softmax_scale))
 
 
 class SelfAttention(nn.Module):
@@ -165,6 +185,10 @@ class SelfAttention(nn.Module):
     def forward(self, hidden_states, attention_mask=None, rotary_pos_emb=None, packed_seq_params=None, **_):
         qkv, _ = self.linear_qkv(hidden_states)  # [s, b, ng*(qpg+2)*d]
         s, b, _w = qkv.shape
+        if self.q_layernorm is None and (rotary_pos_emb is None or self.fused_rope):
+            ctx = self.core_attention.packed(qkv, rotary_pos_emb, self.ng, self.qpg, attention_mask, packed_seq_params)
+            if ctx is not None:
+                return self.linear_proj(ctx)
         if rotary_pos_emb is not None and self.q_layernorm is None and self.fused_rope and qkv.is_contiguous():
             cos, sin = rotary_pos_emb
             qkv = _PackedRope.apply(qkv, cos, sin, self.ng, self.qpg, self.d, self.config.rotary_interleaved)

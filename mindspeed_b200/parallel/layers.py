@@ -21,6 +21,7 @@ pipeline schedule can place them where they hide communication.
 from __future__ import annotations
 
 import math
+import threading
 from typing import Callable, Optional
 
 import torch
@@ -352,6 +353,35 @@ class VocabUtility:
         return VocabUtility.vocab_range_from_per_partition_vocab_size(divide(global_vocab, world_size), rank, world_size)
 
 
+class _EmbeddingFn(torch.autograd.Function):
+    """Embedding lookup whose gradient rows are added straight into the fp32 ``weight.main_grad`` (the accumulation fusion of the
+    linear layers: no dense gradient, the data-parallel wrapper is told through ``weight._main_grad_ready_cb``).  A table may be
+    looked up several times before backward (multi-token prediction): the wrapper is told once no lookup is outstanding, and starts
+    a bucket it was never told about when it finishes the step."""
+    lock = threading.Lock()
+
+    @staticmethod
+    def forward(ctx, ids, weight):
+        ctx.save_for_backward(ids, weight)
+        with _EmbeddingFn.lock:
+            weight.lookups_in_flight = getattr(weight, "lookups_in_flight", 0) + 1
+        return F.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, dout):
+        from ..ops.permute import add_rows_
+        ids, weight = ctx.saved_tensors
+        add_rows_(weight.main_grad, ids.reshape(-1).long().contiguous(), dout.reshape(-1, dout.shape[-1]).contiguous())
+        weight.grad_added_to_main_grad = True
+        with _EmbeddingFn.lock:
+            weight.lookups_in_flight -= 1
+            last = weight.lookups_in_flight <= 0
+        cb = getattr(weight, "_main_grad_ready_cb", None)
+        if cb is not None and last:
+            cb(weight)
+        return None, None
+
+
 class VocabParallelEmbedding(nn.Module):
     """Embedding split along the vocabulary.  Out-of-range ids are masked to row 0 and their
     output rows zeroed before the reduction (reference: mindspeed/core/tensor_parallel/vocab_parallel/vocab_parallel.py:22-56)."""
@@ -367,6 +397,7 @@ class VocabParallelEmbedding(nn.Module):
             num_embeddings, self.rank, self.world)
         self.num_embeddings_per_partition = self.vocab_end_index - self.vocab_start_index
         self.deterministic_mode = config.deterministic_mode
+        self.fuse_grad = bool(config.gradient_accumulation_fusion) and config.optimization_level >= 1
         dev = None if config.use_cpu_initialization or not torch.cuda.is_available() else torch.cuda.current_device()
         self.weight = nn.Parameter(torch.empty(self.num_embeddings_per_partition, embedding_dim, device=dev,
                                                dtype=config.params_dtype))
@@ -381,13 +412,23 @@ class VocabParallelEmbedding(nn.Module):
             masked = (input_ - self.vocab_start_index).masked_fill(mask, 0)
         else:
             masked = input_
-        out = F.embedding(masked, self.weight)
+        out = _EmbeddingFn.apply(masked, self.weight) if self._fused(masked) else F.embedding(masked, self.weight)
         if self.world > 1:
             out = out.masked_fill(mask.unsqueeze(-1), 0.0)
         if self.reduce_scatter_embeddings:
             out = out.transpose(0, 1).contiguous()  # [b,s,h] -> [s,b,h]
             return M.reduce_scatter_to_sequence_parallel_region(out, self.tp_group)
         return M.reduce_from_tensor_model_parallel_region(out, self.tp_group)
+
+    def _fused(self, ids):
+        """Whether the gradient goes straight into ``main_grad``: not for a weight that the output layer shares (its two gradients
+        meet in autograd), nor where the sums have to come out the same in every run."""
+        w = self.weight
+        main = getattr(w, "main_grad", None)
+        return (self.fuse_grad and w.is_cuda and w.requires_grad and torch.is_grad_enabled() and not self.deterministic_mode
+                and not torch.are_deterministic_algorithms_enabled() and not getattr(w, "shared_embedding", False)
+                and torch.is_tensor(main) and main.dtype == torch.float32 and main.is_contiguous() and main.shape == w.shape
+                and w.dtype in (torch.bfloat16, torch.float16, torch.float32) and ids.numel() > 0)
 
     def sharded_state_dict(self, prefix="", sharded_offsets=(), metadata=None):
         from ..checkpointing.sharded import make_tp_sharded_tensors

@@ -49,3 +49,18 @@ def test_scatter_add_rows(n, rows, cols, weighted, dtype):
     assert got.dtype == dtype
     tol = 4e-3 if dtype == torch.bfloat16 else 3e-5
     assert ((got.double() - want).abs() <= tol * want.abs() + 3e-5 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("n,rows,cols", [(1, 1, 8), (300, 7, 264), (5000, 4096, 1536), (64, 3, 133)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_add_rows_into_fp32_table(n, rows, cols, dtype):
+    """fp32 sums of at most n terms in any order: n * 2^-24 of the sum of magnitudes."""
+    from mindspeed_b200.ops.permute import add_rows_
+    torch.manual_seed(n)
+    src = torch.randn(n, cols, device="cuda").to(dtype)
+    idx = torch.randint(0, rows, (n,), device="cuda")
+    out = torch.randn(rows, cols, device="cuda")
+    want = out.double().index_add(0, idx, src.double())
+    size = out.double().abs().index_add(0, idx, src.double().abs())
+    add_rows_(out, idx, src)
+    assert ((out.double() - want).abs() <= (n + 1) * 2.0 ** -24 * size).all()

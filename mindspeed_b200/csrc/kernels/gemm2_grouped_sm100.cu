@@ -102,10 +102,12 @@ struct TileCursor {
       start = offs[e]; end = offs[e + 1];
       cnt = tiles_of(start, end);
     }
-    const int r = t - first;
-    // n fastest inside an expert's m block row so pairs running together share the A rows; weights of one expert stay hot in L2
-    m_blk = r / num_n;
-    n_blk = r - m_blk * num_n;
+    // m fastest inside groups of 8 block rows: the pairs that run together cover about 8 x 9 tiles, so both operands of a wave stay
+    // in L2 and every column panel (a weight's, or dY's in the weight gradient) comes from memory once per group.  With n fastest
+    // a panel of 58 - 235 MB an expert was streamed again for every block row.
+    const int r = t - first, num_m = cnt / num_n, g = r / (8 * num_n), rr = r - g * 8 * num_n, gsz = min(num_m - g * 8, 8);
+    n_blk = rr / gsz;
+    m_blk = g * 8 + (rr - n_blk * gsz);
     t += stride;
     return true;
   }

@@ -6,7 +6,7 @@ import ctypes
 import torch
 
 from . import loader
-from ._dtypes import code
+from ._dtypes import CODE, code
 
 
 class _Gather(torch.autograd.Function):
@@ -75,3 +75,43 @@ def add_rows_(out, idx, src):
     loader.check(L.msb_add_rows_f32(loader.p(src), loader.p(idx), loader.p(out), ctypes.c_longlong(idx.numel()), src.shape[1],
                                     code(src.dtype), ctypes.c_void_p(loader.stream_ptr())), "add_rows_f32")
     return out
+
+
+class _RouteTables(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, probs, routing_map, rows):
+        L = loader.require_lib()
+        T, E = routing_map.shape
+        probs = probs.contiguous()
+        counts = torch.empty(E, dtype=torch.int64, device=probs.device)
+        idx = torch.zeros(rows, dtype=torch.int64, device=probs.device)
+        row_prob = torch.zeros(rows, dtype=probs.dtype, device=probs.device)
+        loader.check(L.msb_moe_route(loader.p(routing_map.contiguous()), loader.p(probs), loader.p(counts), loader.p(idx), loader.p(row_prob),
+                                     ctypes.c_longlong(T), E, ctypes.c_longlong(rows), code(probs.dtype),
+                                     ctypes.c_void_p(loader.stream_ptr())), "moe_route")
+        ctx.save_for_backward(idx, counts)
+        ctx.shape = (T, E)
+        ctx.mark_non_differentiable(idx, counts)
+        return idx, row_prob, counts
+
+    @staticmethod
+    def backward(ctx, _didx, g, _dcounts):
+        idx, counts = ctx.saved_tensors
+        L = loader.require_lib()
+        T, E = ctx.shape
+        g = g.contiguous()
+        dprobs = torch.empty(T, E, dtype=g.dtype, device=g.device)
+        loader.check(L.msb_moe_route_bwd(loader.p(g), loader.p(idx), loader.p(counts), loader.p(dprobs), ctypes.c_longlong(T), E,
+                                         ctypes.c_longlong(idx.numel()), code(g.dtype), ctypes.c_void_p(loader.stream_ptr())), "moe_route_bwd")
+        return dprobs, None, None
+
+
+def route_supports(probs, routing_map) -> bool:
+    return (loader.use_kernels(probs) and routing_map.is_cuda and routing_map.dtype == torch.bool and routing_map.dim() == 2
+            and probs.shape == routing_map.shape and probs.dtype in CODE and routing_map.numel() > 0)
+
+
+def route_tables(probs, routing_map, rows):
+    """probs / routing_map [T, E], ``rows`` = number of entries of the map -> (token of every dispatched row, expert after expert and
+    inside an expert by token [rows]; its probability [rows], differentiable; rows per expert [E]), all on the device."""
+    return _RouteTables.apply(probs, routing_map, rows)

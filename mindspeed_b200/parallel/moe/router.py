@@ -102,6 +102,8 @@ class TopKRouter(nn.Module):
             sg = torch.sigmoid(logits.float())
             scores_for_loss = sg / (sg.sum(-1, keepdim=True) + 1e-20)
         probs = self._aux(scores_for_loss, rmap, tpe, probs, seq_shape)
+        if cfg.moe_expert_capacity_factor is None:
+            rmap.rows_per_token = self.topk          # no token was dropped: the dispatcher knows its row count without asking the device
         return probs, rmap
 
     def update_expert_bias(self):

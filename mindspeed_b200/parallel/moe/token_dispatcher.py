@@ -150,8 +150,16 @@ class MoEAlltoAllTokenDispatcher(MoETokenDispatcher):
         self.hidden_shape = hidden.shape
         h = hidden.reshape(-1, hidden.shape[-1])
         self.routing_map, self.probs = routing_map, probs
-        tokens_per_expert = self.preprocess(routing_map)
         self.restore_shape = h.shape
+        per_token = getattr(routing_map, "rows_per_token", None)
+        if per_token is not None and self.ep_size == 1 and self.fused_permute:
+            from ...ops.permute import gather_rows, route_supports, route_tables
+            if route_supports(probs, routing_map):
+                # every expert is here and every token has ``per_token`` rows: tables and counts stay on the device
+                self.input_splits = self.output_splits = self.chunk_sizes = None
+                self.sorted_indices, pprobs, tokens_per_expert = route_tables(probs, routing_map, h.shape[0] * per_token)
+                return gather_rows(h, self.sorted_indices), tokens_per_expert, pprobs
+        tokens_per_expert = self.preprocess(routing_map)
         permuted, self.sorted_indices = permute(h, routing_map, fused=self.fused_permute)
         pprobs = probs.t().contiguous().masked_select(routing_map.t().contiguous())
         if self.ep_size > 1:

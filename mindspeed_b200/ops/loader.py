@@ -63,7 +63,9 @@ def reset_launch_count() -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle.  Every launch asks for it: the two lookups below take 0.2 us where
+    ``torch.cuda.current_stream()`` takes 8 (it builds a Stream object and looks for devices through the environment)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def check(rc: int, what: str):

@@ -38,6 +38,7 @@ struct Fwd2Params {
   int sq, sk, b, nq, nkv;
   int causal;
   int q_offset;                    // key index visible to query row r is <= r + q_offset
+  int group;                       // (batch, head) pairs whose CTAs are numbered together
   float scale_log2;                // softmax_scale * log2(e)
   unsigned int* status;
 };
@@ -92,9 +93,14 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
   uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(base_ptr + Fwd2Smem::BAR_OFF + 8 * 17);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heavy (late) query tiles first so the causal triangle balances across the grid
-  const int m_blk = (p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
-  const int head = blockIdx.y, batch = blockIdx.z;
+  // (batch, head) pairs in groups of p.group; inside a group the query tiles that see most keys first and the heads fastest, so that
+  // the last CTAs to start are short ones of several heads
+  const int n_m = (p.sq + 2 * FB - 1) / (2 * FB), bh_all = p.b * p.nq;
+  const int grp = (int)(blockIdx.x / (unsigned)(p.group * n_m)), first_bh = grp * p.group, in_grp = min(bh_all - first_bh, p.group);
+  const int rank = (int)(blockIdx.x - (unsigned)(grp * p.group * n_m));
+  const int m_rank = rank / in_grp, bh = first_bh + (rank - m_rank * in_grp);
+  const int m_blk = p.causal ? n_m - 1 - m_rank : m_rank;
+  const int batch = bh / p.nq, head = bh - batch * p.nq;
   const int kv_head = head / (p.nq / p.nkv);
   const int q0 = m_blk * 2 * FB;
   const int n_all = (p.sk + FB - 1) / FB;
@@ -393,7 +399,16 @@ MSB_API int msb_flash_fwd2(const void* q, const void* k, const void* v, void* o,
     if (e != cudaSuccess) { msb_set_error("flash_fwd2: cannot set dynamic shared memory: %s", cudaGetErrorString(e)); return 1; }
     attr = true;
   }
-  dim3 grid((sq + 2 * FB - 1) / (2 * FB), nq, b);
+  // A group is as many heads as have their K and V in half of L2 (48 MB): every CTA that runs at a time then streams from L2, and the
+  // group is wide enough that its shortest CTAs end the launch.  s = 4096, 32 / 8 heads, one head after the other: an SM was busy for
+  // three quarters of the launch.
+  const int rep = nq / nkv, n_m = (sq + 2 * FB - 1) / (2 * FB);
+  const long long kv_heads = (48ll << 20) / ((long long)sk * FD * 4), bh = (long long)b * nq;
+  const long long ctas = bh * n_m;
+  MSB_REQUIRE(ctas <= 0x7fffffffll, "flash_fwd2: grid too large (%lld)", ctas);
+  const long long want = (kv_heads < 1 ? 1 : kv_heads) * rep;
+  p.group = (int)(want < bh ? want : bh);
+  dim3 grid((unsigned)ctas);
   flash_fwd2_sm100_kernel<<<grid, FWD_THREADS, Fwd2Smem::TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("flash_fwd2_sm100");
   return 0;

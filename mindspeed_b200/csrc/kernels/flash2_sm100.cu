@@ -8,8 +8,10 @@
 //   warp 9              MMA issuer (one thread):  S_t = Q_t K_j^T,  O_t += P_t V_j.  Issue order
 //                       S0 S1 | PV0 S0' | PV1 S1' | ...   so tile t's softmax overlaps the other tile's MMAs
 //   warps 0-3 / 4-7     softmax of tile 0 / tile 1, one thread per query row: row maximum (four chains of three-input maxima), exp2,
-//                       row sum, P -> TMEM.  They hold a whole score row per thread (setmaxnreg).  The first 96 keys' probabilities
-//                       are handed to the MMA before the last 32 are computed.  s = 8192, 32 / 8 heads, causal: 573 -> 521 us.
+//                       row sum, P -> TMEM.  They hold a whole score row per thread (setmaxnreg).
+//   The issuing thread is what bounds it, a softmax warp waits a third of the time: a barrier costs it 75 to 150 cycles, done or
+//   not.  One commit frees K and V, the scores' commit stands for P V as well, descriptors are one addition each.  s = 8192, 32 / 8
+//   heads, causal: 573 us at first, 521 with the softmax above, 487 with the heaviest tiles first, 468 with this issue.
 //                       O stays in tensor memory; it is rescaled only when the running maximum grew by more than 2^8
 //                       since the last rescale (the stale maximum is used for P meanwhile, which stays within range),
 //                       so most key tiles never touch O.
@@ -28,7 +30,6 @@ constexpr int FD = 128;                   // head dim
 constexpr int TILE_BYTES = FB * FD * 2;   // 32 KB
 constexpr int HALF_BYTES = FB * 128;      // one 64-wide column block: 128 rows x 128 B
 constexpr float RESCALE_THRESHOLD = 8.f;  // log2 units
-constexpr int P_HEAD = 96;                // keys of a tile whose probabilities are handed to the MMA first
 
 struct Fwd2Params {
   CUtensorMap tmQ;                 // dims {d, head of the group, group, batch, seq}: the heads of a packed QKV activation are not evenly spaced
@@ -82,15 +83,12 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
   const uint32_t bar = base + Fwd2Smem::BAR_OFF;
   const uint32_t q_full = bar;
   auto k_full = [&](int s) { return bar + 8u * (1 + s); };
-  auto k_empty = [&](int s) { return bar + 8u * (3 + s); };
-  auto v_full = [&](int s) { return bar + 8u * (5 + s); };
-  auto v_empty = [&](int s) { return bar + 8u * (7 + s); };
-  auto s_full = [&](int t) { return bar + 8u * (9 + t); };
-  auto p_full = [&](int t) { return bar + 8u * (11 + t); };
-  auto p_tail = [&](int t) { return bar + 8u * (13 + t); };
-  auto pv_done = [&](int t) { return bar + 8u * (15 + t); };
-  const uint32_t tmem_slot = bar + 8u * 17;
-  uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(base_ptr + Fwd2Smem::BAR_OFF + 8 * 17);
+  auto v_full = [&](int s) { return bar + 8u * (3 + s); };
+  auto s_full = [&](int t) { return bar + 8u * (5 + t); };
+  auto p_full = [&](int t) { return bar + 8u * (7 + t); };
+  auto kv_free = [&](int s) { return bar + 8u * (9 + s); };
+  const uint32_t o_done = bar + 8u * 11, tmem_slot = bar + 8u * 12;
+  uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(base_ptr + Fwd2Smem::BAR_OFF + 8 * 12);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (batch, head) pairs in groups of p.group; inside a group the query tiles that see most keys first and the heads fastest, so that
@@ -120,15 +118,17 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
-    for (int t = 0; t < 2; ++t) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 4); mbar_init(p_tail(t), 4); mbar_init(pv_done(t), 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(k_full(s), 1); mbar_init(v_full(s), 1); }
+    for (int t = 0; t < 2; ++t) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 4); }
+    mbar_init(kv_free(0), 1); mbar_init(kv_free(1), 1); mbar_init(o_done, 1);
     mbar_fence_init();
   }
   if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot_ptr;
+  constexpr uint32_t tmem_base = 0;          // all 512 columns are ours
+  if (*tmem_slot_ptr != tmem_base && threadIdx.x == 0) atomicCAS(p.status, 0u, 0x301u);
 
   // registers of the launch: 384 x 168 = 64512; the two softmax warpgroups hold a whole score row per thread
   if (warp >= 8) {       // warps 10 and 11 only complete the warpgroup that gives registers away
@@ -143,20 +143,20 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
         tma_load_5d(qs, &p.tmQ, q_full, 0, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
         tma_load_5d(qs + HALF_BYTES, &p.tmQ, q_full, 64, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
       }
-      bool ok = true;
-      for (int j = 0; j < n_max && ok; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (uint32_t)((j >> 1) & 1);
-        if (!mbar_wait(k_empty(s), ph ^ 1u, p.status, 0x310u)) { ok = false; break; }
-        mbar_arrive_expect_tx(k_full(s), TILE_BYTES);
-        const uint32_t ks = base + Fwd2Smem::K_OFF + s * TILE_BYTES;
-        tma_load_4d(ks, &p.tmK, k_full(s), 0, kv_head, batch, j * FB);
-        tma_load_4d(ks + HALF_BYTES, &p.tmK, k_full(s), 64, kv_head, batch, j * FB);
-        if (!mbar_wait(v_empty(s), ph ^ 1u, p.status, 0x311u)) { ok = false; break; }
-        mbar_arrive_expect_tx(v_full(s), TILE_BYTES);
-        const uint32_t vs = base + Fwd2Smem::V_OFF + s * TILE_BYTES;
-        tma_load_4d(vs, &p.tmV, v_full(s), 0, kv_head, batch, j * FB);
-        tma_load_4d(vs + HALF_BYTES, &p.tmV, v_full(s), 64, kv_head, batch, j * FB);
+      auto load = [&](uint32_t dst, const CUtensorMap* tm, uint32_t full, int j) {
+        mbar_arrive_expect_tx(full, TILE_BYTES);
+        tma_load_4d(dst, tm, full, 0, kv_head, batch, j * FB);
+        tma_load_4d(dst + HALF_BYTES, tm, full, 64, kv_head, batch, j * FB);
+      };
+      auto load_k = [&](int j) { if (j < n_max) load(base + Fwd2Smem::K_OFF + (j & 1) * TILE_BYTES, &p.tmK, k_full(j & 1), j); };
+      auto load_v = [&](int j) { if (j < n_max) load(base + Fwd2Smem::V_OFF + (j & 1) * TILE_BYTES, &p.tmV, v_full(j & 1), j); };
+      load_k(0); load_v(0); load_k(1); load_v(1);
+      // kv_free(c & 1): the scores of key tile c and P V of tile c - 1 are done, so K_c and V_c-1 may be overwritten.  Two barriers in
+      // turn: the one after next needs tiles that are only loaded here, so no phase can pass unseen.
+      for (int c = 0; c + 1 < n_max; ++c) {
+        if (!mbar_wait(kv_free(c & 1), (uint32_t)((c >> 1) & 1), p.status, 0x310u)) break;
+        if (c > 0) load_v(c + 1);
+        load_k(c + 2);
       }
     }
    } else if (warp == 9) {
@@ -164,59 +164,53 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
     if (lane == 0 && n_max > 0) {
       constexpr uint32_t idesc_qk = make_idesc_f16(128, 128, 1, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc_f16(128, 128, 1, 0, 1);
+      // descriptors of tile 0 / stage 0; an address grows by 16-byte units in the low word
+      const uint64_t qd = make_smem_desc(base + Fwd2Smem::Q_OFF, 0, 1024), kd = make_smem_desc(base + Fwd2Smem::K_OFF, 0, 1024);
+      const uint64_t vd = make_smem_desc(base + Fwd2Smem::V_OFF, HALF_BYTES, 1024);
+      auto wait = [&](uint32_t b, uint32_t parity, unsigned int code) {
+        const bool ok = mbar_wait(b, parity, p.status, code);
+        tc_fence_after();
+        return ok;
+      };
       auto issue_s = [&](int t, int j) {
-        const uint32_t qs = base + Fwd2Smem::Q_OFF + t * TILE_BYTES, ks = base + Fwd2Smem::K_OFF + (j & 1) * TILE_BYTES;
-        const uint32_t tS = tmem_base + (uint32_t)(t * 128);
+        const uint64_t q0d = qd + (uint64_t)(t * (TILE_BYTES >> 4)), k0d = kd + (uint64_t)((j & 1) * (TILE_BYTES >> 4));
 #pragma unroll
         for (int k = 0; k < FD / 16; ++k) {
-          const uint32_t off = (uint32_t)((k >> 2) * HALF_BYTES + (k & 3) * 32);
-          umma_f16(tS, make_smem_desc(qs + off, 0, 1024), make_smem_desc(ks + off, 0, 1024), idesc_qk, k ? 1u : 0u);
+          const uint64_t off = (uint64_t)(((k >> 2) * HALF_BYTES + (k & 3) * 32) >> 4);
+          umma_f16(tmem_base + (uint32_t)(t * 128), q0d + off, k0d + off, idesc_qk, k ? 1u : 0u);
         }
-        umma_commit(s_full(t));
+        umma_commit(s_full(t));       // completes after everything issued before: P V of the last key tile is in O as well
       };
-      auto issue_pv = [&](int t, int j, int k0, int k1) {
-        const uint32_t vs = base + Fwd2Smem::V_OFF + (j & 1) * TILE_BYTES;
+      auto issue_pv = [&](int t, int j) {
+        const uint64_t v0d = vd + (uint64_t)((j & 1) * (TILE_BYTES >> 4));
         const uint32_t tP = tmem_base + (uint32_t)(t * 128), tO = tmem_base + 256u + (uint32_t)(t * 128);
 #pragma unroll
-        for (int k = k0; k < k1; ++k) {
-          const uint64_t bdesc = make_smem_desc(vs + (uint32_t)(k * 16 * 128), HALF_BYTES, 1024);   // MN-major: 16 keys = 2048 B
-          umma_f16_ts(tO, tP + (uint32_t)(k * 8), bdesc, idesc_pv, (j | k) ? 1u : 0u);               // 16 bf16 of P = 8 columns
-        }
+        for (int k = 0; k < FB / 16; ++k)      // MN-major: 16 keys = 2048 B; 16 bf16 of P = 8 columns
+          umma_f16_ts(tO, tP + (uint32_t)(k * 8), v0d + (uint64_t)(k * (16 * 128 >> 4)), idesc_pv, (j | k) ? 1u : 0u);
       };
-      bool ok = mbar_wait(q_full, 0, p.status, 0x320u);
-      if (ok) ok = mbar_wait(k_full(0), 0, p.status, 0x321u);
+      bool ok = wait(q_full, 0, 0x320u);
+      if (ok) ok = wait(k_full(0), 0, 0x321u);
       if (ok) {
-        tc_fence_after();
-        for (int t = 0; t < 2; ++t) if (n_t[t] > 0) issue_s(t, 0);
-        umma_commit(k_empty(0));
+        if (n_t[0] > 0) issue_s(0, 0);
+        if (n_t[1] > 0) issue_s(1, 0);
+        umma_commit(kv_free(0));
       }
       for (int j = 0; j < n_max && ok; ++j) {
         const uint32_t ph = (uint32_t)((j >> 1) & 1), jp = (uint32_t)(j & 1);
-        if (!mbar_wait(v_full(j & 1), ph, p.status, 0x322u)) { ok = false; break; }
-        bool k_next_ready = false;
-        for (int t = 0; t < 2 && ok; ++t) {
+        if (!(ok = wait(v_full(j & 1), ph, 0x322u))) break;
+        if (j + 1 < n_max && !(ok = wait(k_full((j + 1) & 1), (uint32_t)(((j + 1) >> 1) & 1), 0x324u))) break;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
           if (j < n_t[t]) {
-            if (!mbar_wait(p_full(t), jp, p.status, 0x323u)) { ok = false; break; }
-            tc_fence_after();
-            issue_pv(t, j, 0, P_HEAD / 16);
-            if (!mbar_wait(p_tail(t), jp, p.status, 0x325u)) { ok = false; break; }
-            tc_fence_after();
-            issue_pv(t, j, P_HEAD / 16, FB / 16);
-            umma_commit(pv_done(t));
+            if (!(ok = wait(p_full(t), jp, 0x323u))) break;
+            issue_pv(t, j);
           }
-          if (j + 1 < n_t[t]) {
-            if (!k_next_ready) {
-              if (!mbar_wait(k_full((j + 1) & 1), (uint32_t)(((j + 1) >> 1) & 1), p.status, 0x324u)) { ok = false; break; }
-              tc_fence_after();
-              k_next_ready = true;
-            }
-            issue_s(t, j + 1);
-          }
+          if (j + 1 < n_t[t]) issue_s(t, j + 1);
         }
         if (!ok) break;
-        umma_commit(v_empty(j & 1));
-        if (j + 1 < n_max) umma_commit(k_empty((j + 1) & 1));
+        umma_commit(kv_free((j + 1) & 1));
       }
+      if (ok) umma_commit(o_done);
     }
    }
   } else {
@@ -263,9 +257,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
       if (__any_sync(0xffffffffu, grow)) {
         const float m_new = fmaxf(m_used, m_tile2);
         const float alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - m_new);
-        if (j > 0) {
-          if (!mbar_wait(pv_done(t), jp ^ 1u, p.status, 0x331u)) { ok = false; break; }   // P V of tile j-1 has landed in O
-          tc_fence_after();
+        if (j > 0) {                             // the scores' commit covered P V of tile j - 1, which is in O
 #pragma unroll 1
           for (int c = 0; c < FD; c += 32) {
             uint32_t r[32];
@@ -281,8 +273,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
         m_used = m_new;
       }
       const float m_ref = (m_used == -INFINITY) ? 0.f : m_used;
-      // probabilities -> packed bf16 over the first 64 columns of S, row sum (masked scores are -inf -> 0).  The first P_HEAD
-      // keys are handed over as soon as they are stored, so P V starts while the last quarter is still being computed.
+      // probabilities -> packed bf16 over the first 64 columns of S, row sum (masked scores are -inf -> 0)
       const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), nref2 = pack_f32x2(-m_ref, -m_ref);
       uint64_t sum2[2] = {0ull, 0ull};
 #pragma unroll
@@ -298,13 +289,11 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
           pk[i] = pack_bf16(pa, pb);
         }
         tmem_st_32x16(tS + (uint32_t)(c >> 1), pk);
-        if (c + 32 == P_HEAD || c + 32 == FB) {
-          tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(c + 32 == FB ? p_tail(t) : p_full(t));   // one arrival per warp: 128 on one barrier would serialise
-        }
       }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full(t));       // one arrival per warp: 128 on one barrier would serialise
       float l0, l1, l2, l3;
       unpack_f32x2(sum2[0], l0, l1);
       unpack_f32x2(sum2[1], l2, l3);
@@ -312,7 +301,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
     }
     // ---- epilogue of this tile ----
     if (n_kv > 0) {
-      if (ok) ok = mbar_wait(pv_done(t), (uint32_t)((n_kv - 1) & 1), p.status, 0x332u);
+      if (ok) ok = mbar_wait(o_done, 0, p.status, 0x332u);
       tc_fence_after();
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       uint8_t* o_row = base_ptr + Fwd2Smem::Q_OFF + t * TILE_BYTES + row * 128;   // the tile's Q buffer: no MMA reads it any more
@@ -438,7 +427,7 @@ MSB_API int msb_flash_fwd2(const void* q, const void* k, const void* v, void* o,
 //   warps 10-13   dQ: tensor memory -> softmax scale -> staging -> TMA reduce-add into the fp32 dQ
 // Bound: shared memory moves 490 KB per 128 x 128 tile (operands 290, TMA writes 64, dS 32, dQ staging in and out 128), 3840 cycles at
 // 128 B a cycle, beside 2560 cycles of MMA.  Measured at s = 8192, 32 / 8 heads, causal: 2173 us with one tile in flight and four
-// compute warps, 1251 us so.
+// compute warps, 1251 us so, 1201 with dQ's columns handed back before its first quarter is sent.
 // reference semantics: the attention grad op of the reference, mindspeed/ops/csrc/cann/fusion_attention_v2.cpp:431-439.
 // =====================================================================================================================
 namespace {
@@ -785,7 +774,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
         uint32_t r[3][32];                               // d columns 32k .. 32k+31 of this lane's query row; the last 32 reuse r[0]
         const uint32_t tQ = tDPT + lane_addr;
         const int qr = i * FB + q * 32;                  // first query row of this warp's block
-        auto put = [&](const uint32_t* v, int c) {       // 32 columns -> 4 KB slot c & 1 -> reduce-add
+        auto put = [&](const uint32_t* v, int c) {       // 32 columns -> 4 KB slot c & 1
           if (lane == 0) tma_store_wait_read<1>();       // the reduce-add before the last one has read this slot
           __syncwarp();
           uint8_t* srow = st_ptr + (c & 1) * 4096;
@@ -794,6 +783,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
             *reinterpret_cast<float4*>(srow + ((k ^ (lane & 7)) << 4)) =
                 make_float4(__uint_as_float(v[4 * k]) * p.scale, __uint_as_float(v[4 * k + 1]) * p.scale,
                             __uint_as_float(v[4 * k + 2]) * p.scale, __uint_as_float(v[4 * k + 3]) * p.scale);
+        };
+        auto send = [&](int c) {
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
@@ -801,6 +792,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
             tma_store_commit();
           }
         };
+        // three quarters fit the registers; the first leaves for shared memory at once (its slot has long been read), the last takes
+        // its place, and dQ's columns are free
         tmem_ld_32x32(tQ, r[0]);
         tmem_ld_32x32(tQ + 32u, r[1]);
         tmem_ld_32x32(tQ + 64u, r[2]);
@@ -811,9 +804,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) flash_bwd_sm100_kernel(const _
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(dq_drained);          // the MMA thread may overwrite dQ with the next dP^T
+        send(0);
         put(r[1], 1);
+        send(1);
         put(r[2], 2);
+        send(2);
         put(r[0], 3);
+        send(3);
         if (++i == n_q) { i = i_start; ++head; }
       }
       if (lane == 0) tma_store_wait<0>();

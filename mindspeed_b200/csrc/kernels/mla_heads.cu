@@ -3,7 +3,7 @@
 //
 //   forward   q [T, n, nope + rope], kv [T, n, nope + vd], k_pe [T, rope]  ->  qf [T, n, nope + rope] (last `rope` rotated),
 //             kf [T, n, nope + rope] = (k of kv | rotated k_pe, the same for every head), v [T, n, vd]
-//   backward  dqf, dkf, dv -> dq, dkv and dk_pe (summed over the heads in fp32, in head order, then rotated back and rounded once)
+//   backward  dqf, dkf, dv -> dq, dkv and dk_pe (summed over the heads in fp32, in a fixed order, then rotated back and rounded once)
 //
 // Bound by memory: every value is read and written once.  A block owns a token, so that k_pe, the angles and the sum over heads
 // stay on the SM; 16-byte accesses.  (As slices, concatenations and element-wise rotations in PyTorch the same work made 12
@@ -45,10 +45,38 @@ __device__ __forceinline__ void rot16(float* u, float* w, const float* cos, cons
 __device__ __forceinline__ int first_col(int j, const MlaDims& d) { return d.interleaved ? 16 * j : 8 * j; }
 __device__ __forceinline__ int second_col(int j, const MlaDims& d) { return d.interleaved ? 16 * j + 8 : d.rope / 2 + 8 * j; }
 
-template <typename T>
-__device__ __forceinline__ void copy8(T* dst, const T* src) { Vec8<T> t; t.load(src); t.store(dst); }
+// n rows (heads) of w8 vectors of eight values, from stride ss to stride ds (elements); four loads in flight a thread
+template <typename T, int W8>
+__device__ __forceinline__ void copy_heads(T* __restrict__ dst, long long ds, const T* __restrict__ src, long long ss, int n, int w8_) {
+  const int w8 = W8 ? W8 : w8_, total = n * w8;
+  int i = threadIdx.x;
+  for (; i + 3 * (int)blockDim.x < total; i += 4 * blockDim.x) {
+    Vec8<T> t[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { const int j = i + k * (int)blockDim.x, h = j / w8; t[k].load(src + h * ss + 8 * (j - h * w8)); }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { const int j = i + k * (int)blockDim.x, h = j / w8; t[k].store(dst + h * ds + 8 * (j - h * w8)); }
+  }
+  for (; i < total; i += blockDim.x) { const int h = i / w8; Vec8<T> t; t.load(src + h * ss + 8 * (i - h * w8)); t.store(dst + h * ds + 8 * (i - h * w8)); }
+}
+// the rotary part of n heads (src and dst at its first column), p8 groups of eight pairs a head
+template <typename T, int P8>
+__device__ __forceinline__ void rotate_heads(T* __restrict__ dst, long long ds, const T* __restrict__ src, long long ss, const float* c, const float* s,
+                                             const MlaDims& d, bool back) {
+  const int p8 = P8 ? P8 : d.rope / 16;
+  for (int i = threadIdx.x; i < d.n * p8; i += blockDim.x) {
+    const int h = i / p8, j = i - h * p8, a = first_col(j, d), b = second_col(j, d);
+    Vec8<T> x, y;
+    x.load(src + h * ss + a); y.load(src + h * ss + b);
+    float u[8], w[8];
+    x.to_float(u); y.to_float(w);
+    rot16(u, w, c, s, j, d, back);
+    x.from_float(u); y.from_float(w);
+    x.store(dst + h * ds + a); y.store(dst + h * ds + b);
+  }
+}
 
-template <typename T>
+template <typename T, int N8, int R8, int V8>
 __global__ void __launch_bounds__(256) mla_heads_fwd_kernel(const T* __restrict__ q, const T* __restrict__ kv, const T* __restrict__ k_pe,
                                                             Strided sp, const float* __restrict__ cos, const float* __restrict__ sin,
                                                             T* __restrict__ qf, T* __restrict__ kf, T* __restrict__ v, MlaDims d) {
@@ -77,34 +105,20 @@ __global__ void __launch_bounds__(256) mla_heads_fwd_kernel(const T* __restrict_
   const int qk = d.nope + d.rope, kw = d.nope + d.vd;
   const T *q0 = q + t * d.n * qk, *kv0 = kv + t * d.n * kw;
   T *qf0 = qf + t * d.n * qk, *kf0 = kf + t * d.n * qk, *v0 = v + t * d.n * d.vd;
-  // items of a head, 8 columns each: q nope | q pairs (16 columns) | k nope | k rotary | v
-  const int i0 = d.nope / 8, i1 = i0 + pairs8, i2 = i1 + d.nope / 8, i3 = i2 + d.rope / 8, per = i3 + d.vd / 8;
-  for (int i = threadIdx.x; i < d.n * per; i += blockDim.x) {
-    const int h = i / per, k = i - h * per;
-    if (k < i0) {
-      copy8(qf0 + h * qk + 8 * k, q0 + h * qk + 8 * k);
-    } else if (k < i1) {
-      const int j = k - i0, a = d.nope + first_col(j, d), b = d.nope + second_col(j, d);
-      Vec8<T> x, y;
-      x.load(q0 + h * qk + a); y.load(q0 + h * qk + b);
-      float u[8], w[8];
-      x.to_float(u); y.to_float(w);
-      rot16(u, w, c, s, j, d, false);
-      x.from_float(u); y.from_float(w);
-      x.store(qf0 + h * qk + a); y.store(qf0 + h * qk + b);
-    } else if (k < i2) {
-      copy8(kf0 + h * qk + 8 * (k - i1), kv0 + h * kw + 8 * (k - i1));
-    } else if (k < i3) {
-      Vec8<T> x;
-      x.from_float(pe + 8 * (k - i2));
-      x.store(kf0 + h * qk + d.nope + 8 * (k - i2));
-    } else {
-      copy8(v0 + h * d.vd + 8 * (k - i3), kv0 + h * kw + d.nope + 8 * (k - i3));
-    }
+  copy_heads<T, N8>(qf0, qk, q0, qk, d.n, d.nope / 8);
+  copy_heads<T, N8>(kf0, qk, kv0, kw, d.n, d.nope / 8);
+  copy_heads<T, V8>(v0, d.vd, kv0 + d.nope, kw, d.n, d.vd / 8);
+  rotate_heads<T, R8 / 2>(qf0 + d.nope, qk, q0 + d.nope, qk, c, s, d, false);
+  const int r8 = R8 ? R8 : d.rope / 8;
+  for (int i = threadIdx.x; i < d.n * r8; i += blockDim.x) {
+    const int h = i / r8, k = i - h * r8;
+    Vec8<T> x;
+    x.from_float(pe + 8 * k);
+    x.store(kf0 + h * qk + d.nope + 8 * k);
   }
 }
 
-template <typename T>
+template <typename T, int N8, int R8, int V8>
 __global__ void __launch_bounds__(256) mla_heads_bwd_kernel(const T* __restrict__ dqf, Strided sq, const T* __restrict__ dkf, Strided sk,
                                                             const T* __restrict__ dv, Strided sv, const float* __restrict__ cos,
                                                             const float* __restrict__ sin, T* __restrict__ dq, T* __restrict__ dkv,
@@ -121,30 +135,31 @@ __global__ void __launch_bounds__(256) mla_heads_bwd_kernel(const T* __restrict_
   __syncthreads();
   const int pairs8 = d.rope / 16, qk = d.nope + d.rope, kw = d.nope + d.vd;
   T *q0 = dq + t * d.n * qk, *kv0 = dkv + t * d.n * kw;
-  const int i0 = d.nope / 8, i1 = i0 + pairs8, i2 = i1 + d.nope / 8, per = i2 + d.vd / 8;
-  for (int i = threadIdx.x; i < d.n * per; i += blockDim.x) {
-    const int h = i / per, k = i - h * per;
-    if (k < i0) {
-      copy8(q0 + h * qk + 8 * k, dq0 + h * sq.h + 8 * k);
-    } else if (k < i1) {
-      const int j = k - i0, a = d.nope + first_col(j, d), b = d.nope + second_col(j, d);
-      Vec8<T> x, y;
-      x.load(dq0 + h * sq.h + a); y.load(dq0 + h * sq.h + b);
-      float u[8], w[8];
-      x.to_float(u); y.to_float(w);
-      rot16(u, w, c, s, j, d, true);
-      x.from_float(u); y.from_float(w);
-      x.store(q0 + h * qk + a); y.store(q0 + h * qk + b);
-    } else if (k < i2) {
-      copy8(kv0 + h * kw + 8 * (k - i1), dk0 + h * sk.h + 8 * (k - i1));
-    } else {
-      copy8(kv0 + h * kw + d.nope + 8 * (k - i2), dv0 + h * sv.h + 8 * (k - i2));
+  copy_heads<T, N8>(q0, qk, dq0, sq.h, d.n, d.nope / 8);
+  copy_heads<T, N8>(kv0, kw, dk0, sk.h, d.n, d.nope / 8);
+  copy_heads<T, V8>(kv0 + d.nope, kw, dv0, sv.h, d.n, d.vd / 8);
+  rotate_heads<T, R8 / 2>(q0 + d.nope, qk, dq0 + d.nope, sq.h, c, s, d, true);
+  // sum over heads: eight columns a thread, the heads dealt to `parts` threads a column whose sums meet in a fixed order
+  const int r8 = d.rope / 8, parts = max(1, min(d.n, (int)blockDim.x / r8));
+  for (int i = threadIdx.x; i < r8 * parts; i += blockDim.x) {
+    const int part = i / r8, k = i - part * r8;
+    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int h = part; h < d.n; h += parts) {
+      Vec8<T> x;
+      float f[8];
+      x.load(dk0 + h * sk.h + d.nope + 8 * k);
+      x.to_float(f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sum[e] += f[e];
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) pe[(1 + part) * d.rope + 8 * k + e] = sum[e];
   }
-  for (int i = threadIdx.x; i < d.rope; i += blockDim.x) {             // a column per thread, heads in order
+  __syncthreads();
+  for (int i = threadIdx.x; i < d.rope; i += blockDim.x) {
     float sum = 0.f;
-#pragma unroll 8
-    for (int h = 0; h < d.n; ++h) sum += to_f(dk0[h * sk.h + d.nope + i]);
+    for (int part = 0; part < parts; ++part) sum += pe[(1 + part) * d.rope + i];
     pe[i] = sum;
   }
   __syncthreads();
@@ -178,8 +193,11 @@ MSB_API int msb_mla_heads_fwd(const void* q, const void* kv, const void* k_pe, l
   MlaDims d{n, nope, rope, vd, b, interleaved};
   int rc = check_dims(tokens, d); if (rc) return rc;
   Strided sp{pe_s, pe_b, 0};
-  MSB_DISPATCH_FLOAT(dtype, T, mla_heads_fwd_kernel<T><<<(unsigned)tokens, 256, 3 * rope * sizeof(float), s>>>((const T*)q, (const T*)kv, (const T*)k_pe,
-                     sp, cos, sin, (T*)qf, (T*)kf, (T*)v, d));
+  const bool common = nope == 128 && rope == 64 && vd == 128;      // widths known at compile time: no divisions, unrolled copies
+  MSB_DISPATCH_FLOAT(dtype, T, {
+    auto kern = common ? mla_heads_fwd_kernel<T, 16, 8, 16> : mla_heads_fwd_kernel<T, 0, 0, 0>;
+    kern<<<(unsigned)tokens, 256, 3 * rope * sizeof(float), s>>>((const T*)q, (const T*)kv, (const T*)k_pe, sp, cos, sin, (T*)qf, (T*)kf, (T*)v, d);
+  });
   MSB_CHECK_LAUNCH("mla_heads_fwd");
   return 0;
 }
@@ -192,8 +210,13 @@ MSB_API int msb_mla_heads_bwd(const void* dqf, long long q_s, long long q_b, lon
   MlaDims d{n, nope, rope, vd, b, interleaved};
   int rc = check_dims(tokens, d); if (rc) return rc;
   Strided sq{q_s, q_b, q_h}, sk{k_s, k_b, k_h}, sv{v_s, v_b, v_h};
-  MSB_DISPATCH_FLOAT(dtype, T, mla_heads_bwd_kernel<T><<<(unsigned)tokens, 256, 3 * rope * sizeof(float), s>>>((const T*)dqf, sq, (const T*)dkf, sk,
-                     (const T*)dv, sv, cos, sin, (T*)dq, (T*)dkv, (T*)dk_pe, d));
+  const bool common = nope == 128 && rope == 64 && vd == 128;
+  const int r8 = rope / 8, parts = 256 / r8 < n ? (256 / r8 < 1 ? 1 : 256 / r8) : n;
+  const size_t sh = (size_t)(3 + parts) * rope * sizeof(float);
+  MSB_DISPATCH_FLOAT(dtype, T, {
+    auto kern = common ? mla_heads_bwd_kernel<T, 16, 8, 16> : mla_heads_bwd_kernel<T, 0, 0, 0>;
+    kern<<<(unsigned)tokens, 256, sh, s>>>((const T*)dqf, sq, (const T*)dkf, sk, (const T*)dv, sv, cos, sin, (T*)dq, (T*)dkv, (T*)dk_pe, d);
+  });
   MSB_CHECK_LAUNCH("mla_heads_bwd");
   return 0;
 }

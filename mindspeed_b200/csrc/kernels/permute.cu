@@ -1,7 +1,7 @@
 // MoE token permutation: row gather and (optionally weighted) row scatter-add with fp32 accumulation.
-// The scatter-add runs as a gather: the source rows of every output row are chained into a list (one exchange per source row), then
-// a block per output row walks its list, sums the rows in registers (ascending up to 64 rows, so that the order in which threads
-// run does not show) and writes the result once.  Bound by the read of the source rows.  (As fp32 atomics into a zeroed buffer that
+// The scatter-add runs as a gather: every source row enters its output row's table of eight slots, or a list behind it, then a block
+// per output row sums them in registers (slots in ascending order, so that up to eight the order in which threads run does not
+// show) and writes the result once.  Bound by the read of the source rows.  (As fp32 atomics into a zeroed buffer that
 // was rounded afterwards, 24576 rows of 4096 took 180 us beside 25 us for the passes around it.)
 // reference semantics: npu_moe_token_permute / npu_moe_token_unpermute
 // (mindspeed/ops/csrc/cann/npu_moe_token_permute.cpp, npu_moe_token_unpermute.cpp).
@@ -23,44 +23,66 @@ __global__ void gather_rows_kernel(const T* __restrict__ x, const long long* __r
     }
   }
 }
+constexpr int SLOTS = 8;               // source rows of an output row that are found without walking a list (a token's experts)
 constexpr int CHAIN = 64;              // list entries taken at a time (and put in ascending order)
 
-__global__ void chain_rows_kernel(const long long* __restrict__ idx, long long* __restrict__ head, long long* __restrict__ next, long long n) {
-  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x)
-    next[r] = (long long)atomicExch(reinterpret_cast<unsigned long long*>(head + idx[r]), (unsigned long long)r);
+// scratch of one call, long long each: count [rows] | head of the overflow list [rows] | slots [rows, 8] | next [n]
+struct Chains {
+  long long *count, *head, *slot, *next;
+  __host__ __device__ Chains(long long* p, long long rows) : count(p), head(p + rows), slot(p + 2 * rows), next(p + (2 + SLOTS) * rows) {}
+};
+
+__global__ void chain_rows_kernel(const long long* __restrict__ idx, Chains c, long long n) {
+  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {
+    const long long o = idx[r], pos = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(c.count + o), 1ull);
+    if (pos < SLOTS) c.slot[o * SLOTS + pos] = r;
+    else c.next[r] = (long long)atomicExch(reinterpret_cast<unsigned long long*>(c.head + o), (unsigned long long)r);
+  }
 }
 
 // weight (optional): one factor per source row
 template <typename T>
-__global__ void sum_chains_kernel(const T* __restrict__ src, const float* __restrict__ weight, const long long* __restrict__ head,
-                                  const long long* __restrict__ next, T* __restrict__ out, long long rows, int cols, int vec) {
+__global__ void sum_chains_kernel(const T* __restrict__ src, const float* __restrict__ weight, Chains ch, T* __restrict__ out, long long rows,
+                                  int cols, int vec) {
   __shared__ long long list[CHAIN];
   __shared__ int count;
   for (long long o = blockIdx.x; o < rows; o += gridDim.x) {
     T* dst = out + (size_t)o * cols;
+    const long long n = ch.count[o];
     // columns in chunks of 8 per thread; rows with more source rows than a list holds take several rounds per chunk
     for (int c0 = 0; c0 < cols; c0 += (int)blockDim.x * 8) {
       const int c = c0 + (int)threadIdx.x * 8;
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      long long at = head[o];
+      long long at = n > SLOTS ? ch.head[o] : -1;      // overflow that is still to come
+      bool first = true;
       do {
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (first) {                                   // the slots, every one ranked by its own thread
+          const int k = (int)(n < SLOTS ? n : SLOTS);
+          if ((int)threadIdx.x < k) {
+            const long long mine = ch.slot[o * SLOTS + threadIdx.x];
+            int rank = 0;
+            for (int i = 0; i < k; ++i) rank += ch.slot[o * SLOTS + i] < mine ? 1 : 0;
+            list[rank] = mine;
+          }
+          if (threadIdx.x == 0) count = k;
+        } else if (threadIdx.x == 0) {
           int k = 0;
-          for (; k < CHAIN && at >= 0; ++k, at = next[at]) {
-            int j = k;                                 // ascending
-            for (; j > 0 && list[j - 1] > at; --j) list[j] = list[j - 1];
-            list[j] = at;
+          for (long long w = at; k < CHAIN && w >= 0; ++k, w = ch.next[w]) {
+            int j = k;
+            for (; j > 0 && list[j - 1] > w; --j) list[j] = list[j - 1];
+            list[j] = w;
           }
           count = k;
         }
         __syncthreads();
         const int k = count;
-        if (k == CHAIN) {                              // everyone follows to where thread 0 stands
-          if (threadIdx.x != 0) for (int i = 0; i < CHAIN; ++i) at = next[at];
-        } else {
-          at = -1;
+        if (!first) {                                  // everyone moves on to what the next round takes
+          if (k == CHAIN) { for (int i = 0; i < CHAIN; ++i) at = ch.next[at]; }
+          else at = -1;
         }
+        first = false;
+#pragma unroll 4
         for (int i = 0; i < k; ++i) {
           const long long r = list[i];
           const float w = weight ? weight[r] : 1.f;
@@ -121,21 +143,23 @@ MSB_API int msb_gather_rows(const void* x, const long long* idx, void* out, long
   return 0;
 }
 // out [rows, cols] = for every source row r < n: out[idx[r]] += src[r] * (weight ? weight[r] : 1), summed in fp32; rows that no
-// source row names become zero.  chain: int64 scratch [rows + n].
+// source row names become zero.  chain: int64 scratch [10 rows + n].
 MSB_API int msb_scatter_add_rows(const void* src, const long long* idx, const float* weight, void* out, long long* chain, long long n, long long rows,
                                  int cols, int dtype, cudaStream_t s) {
   if (rows == 0 || cols == 0) return 0;
-  cudaError_t e = cudaMemsetAsync(chain, 0xff, (size_t)rows * sizeof(long long), s);
+  const Chains ch(chain, rows);
+  cudaError_t e = cudaMemsetAsync(ch.count, 0, (size_t)rows * sizeof(long long), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(ch.head, 0xff, (size_t)rows * sizeof(long long), s);
   if (e != cudaSuccess) { msb_set_error("scatter_add_rows: %s", cudaGetErrorString(e)); return 1; }
   if (n > 0) {
     const int cgrid = (int)(((n + 255) / 256) < (long long)msb::num_sms() * 8 ? (n + 255) / 256 : (long long)msb::num_sms() * 8);
-    chain_rows_kernel<<<cgrid, 256, 0, s>>>(idx, chain, chain + rows, n);
+    chain_rows_kernel<<<cgrid, 256, 0, s>>>(idx, ch, n);
     MSB_CHECK_LAUNCH("chain_rows");
   }
   const int vec = (cols % 8 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) ? 1 : 0;
   const int threads = cols >= 4096 ? 512 : cols >= 2048 ? 256 : 128;
   const int grid = (int)(rows < (long long)msb::num_sms() * 32 ? rows : (long long)msb::num_sms() * 32);
-  MSB_DISPATCH_FLOAT(dtype, T, sum_chains_kernel<T><<<grid, threads, 0, s>>>((const T*)src, weight, chain, chain + rows, (T*)out, rows, cols, vec));
+  MSB_DISPATCH_FLOAT(dtype, T, sum_chains_kernel<T><<<grid, threads, 0, s>>>((const T*)src, weight, ch, (T*)out, rows, cols, vec));
   MSB_CHECK_LAUNCH("scatter_add_rows");
   return 0;
 }

@@ -31,7 +31,7 @@ class _Gather(torch.autograd.Function):
 def _scatter(src, idx, rows, weight):
     L = loader.require_lib()
     out = torch.empty(rows, src.shape[1], dtype=src.dtype, device=src.device)
-    chain = torch.empty(rows + idx.numel(), dtype=torch.int64, device=src.device)
+    chain = torch.empty(10 * rows + idx.numel(), dtype=torch.int64, device=src.device)
     loader.check(L.msb_scatter_add_rows(loader.p(src), loader.p(idx), loader.p(weight), loader.p(out), loader.p(chain),
                                         ctypes.c_longlong(idx.numel()), ctypes.c_longlong(rows), src.shape[1], code(src.dtype),
                                         ctypes.c_void_p(loader.stream_ptr())), "scatter_add_rows")

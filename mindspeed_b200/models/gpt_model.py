@@ -127,6 +127,10 @@ class GPTModel(nn.Module):
         mtp_loss = None
         if self.mtp is not None and labels is not None and self.training:
             mtp_loss = self.mtp(hidden, input_ids, position_ids, labels, loss_mask, self, rpe, attention_mask)
+        if labels is None and hidden.shape[1] > 1 and ps.get_tensor_model_parallel_world_size() == 1:
+            # sample-major logits: the hidden states change places before the product, not the (vocabulary / hidden times larger) logits
+            logits, _ = self.output_layer(hidden.transpose(0, 1).contiguous(), weight=weight)
+            return logits
         logits, _ = self.output_layer(hidden, weight=weight)  # [s, b, V/tp]
         if labels is None:
             return logits.transpose(0, 1).contiguous()

@@ -263,6 +263,12 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
+// The same for handing tensor memory back to the pair's issuing thread: what is ordered are tcgen05.ld completions (wait::ld and
+// fence::before_thread_sync), so the release keeps the default CTA scope.  A cluster-scope release waits for every outstanding load of
+// the thread first, an L2 latency per hand-over.
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
 // 2-D tiled load into THIS CTA's shared memory whose byte count is credited to a barrier given by its cluster-wide
 // address (the leader's), so one barrier phase covers both CTAs' halves of a stage.  Plain load: every CTA fetches its own tile.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, uint32_t cluster_bar, int x, int y) {

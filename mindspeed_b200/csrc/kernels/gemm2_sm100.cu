@@ -288,7 +288,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1) gemm2_sm100_
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(lead_tempty[acc]);   // this warp has read its lanes of the accumulator
+      if (lane == 0) mbar_arrive_remote(lead_tempty[acc]);   // this warp has read its lanes of the accumulator
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
     if (lane == 0) tma_store_wait<0>();                 // staging buffers are read and the stores are complete before exit

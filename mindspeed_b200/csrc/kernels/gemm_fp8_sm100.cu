@@ -30,6 +30,11 @@
 using namespace msb;
 using namespace msb::sm100;
 
+namespace msb {
+int gemm2_fp8_blockscaled(const void* A, const float* sA_t, const void* B, const float* sB, void* D, int M, int N, int K, int b_scale_rowwise,
+                          int fmt_a, int fmt_b, int epilogue, long long ldd, unsigned int* status, cudaStream_t s);
+}
+
 namespace {
 
 constexpr int FBM = 128, FBN = 128, FBK = 128;   // FBK in fp8 elements = bytes
@@ -84,7 +89,7 @@ __global__ void __launch_bounds__(320, 1) gemm_fp8_blockscaled_kernel(const __gr
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < FSTAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int a = 0; a < NACC; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 256); }
+    for (int a = 0; a < NACC; ++a) { mbar_init(tfull_bar(a), 1); mbar_init(tempty_bar(a), 8); }
     mbar_fence_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, F_TMEM_COLS); tmem_relinquish(); }
@@ -166,16 +171,21 @@ __global__ void __launch_bounds__(320, 1) gemm_fp8_blockscaled_kernel(const __gr
 #pragma unroll
       for (int c = 0; c < HC; ++c) accum[c] = 0.f;
       const float* sb_blk = p.sB + (long long)(ncol0 / FBN) * num_kb;
-      // scales of the next k-block are fetched while the current one is folded in (a global load per k-block would
-      // otherwise sit on the critical path of every promotion)
-      float sa_next = row_ok ? __ldg(p.sA + row) : 0.f;
-      float sbs_next = p.b_scale_rowwise ? 1.f : __ldg(sb_blk);
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const float sa = sa_next, sbs = sbs_next;
-        if (kb + 1 < num_kb) {
-          sa_next = row_ok ? __ldg(p.sA + (long long)(kb + 1) * p.M + row) : 0.f;
-          if (!p.b_scale_rowwise) sbs_next = __ldg(sb_blk + kb + 1);
-        }
+      // scales are fetched AHEAD k-blocks before they are used: one ahead, the load's latency was the time of a k-block
+      constexpr int AHEAD = 4;
+      auto scale_a = [&](int kb) { return row_ok && kb < num_kb ? __ldg(p.sA + (long long)kb * p.M + row) : 0.f; };
+      auto scale_b = [&](int kb) { return !p.b_scale_rowwise && kb < num_kb ? __ldg(sb_blk + kb) : 1.f; };
+      float sa_q[AHEAD], sb_q[AHEAD];
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) { sa_q[i] = scale_a(i); sb_q[i] = scale_b(i); }
+      for (int kb0 = 0; kb0 < num_kb && alive; kb0 += AHEAD) {
+#pragma unroll
+       for (int u = 0; u < AHEAD; ++u) {                   // a slot keeps its register: moving it would wait for the load
+        const int kb = kb0 + u;
+        if (kb >= num_kb) break;
+        const float sa = sa_q[u], sbs = sb_q[u];
+        sa_q[u] = scale_a(kb + AHEAD);
+        sb_q[u] = scale_b(kb + AHEAD);
         if (!mbar_wait(tfull_bar(acc), acc_phase, p.status, 0x430u)) { alive = false; break; }
         tc_fence_after();
         const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * FBN + cbase);
@@ -212,8 +222,10 @@ __global__ void __launch_bounds__(320, 1) gemm_fp8_blockscaled_kernel(const __gr
           }
         }
         tc_fence_before();
-        mbar_arrive(tempty_bar(acc));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty_bar(acc));     // one arrival per warp: 256 on one barrier serialise
         if (++acc == NACC) { acc = 0; acc_phase ^= 1u; }
+       }
       }
       if (!alive) break;
       if (row_ok) {
@@ -265,6 +277,17 @@ __global__ void __launch_bounds__(320, 1) gemm_fp8_blockscaled_kernel(const __gr
   }
 }
 
+// Whether the 256 x 256 CTA-pair kernel (gemm2_fp8_sm100.cu) takes a plain GEMM: output rows on 16-byte boundaries (TMA stores),
+// row-wise scales of B in 16-byte pieces.  Its tile wants half a wave of CTA pairs: below that the four times as many
+// 128 x 128 tiles of this file fill the chip better.
+bool pair_kernel_fits(const void* D, const float* sB, int M, int N, int b_scale_rowwise, int epilogue, long long ldd) {
+  const long long row_bytes = ldd * (epilogue == FEPI_BF16 ? 2 : 4);
+  if ((reinterpret_cast<uintptr_t>(D) | (uintptr_t)row_bytes) & 15) return false;
+  if (b_scale_rowwise && ((N & 3) || (reinterpret_cast<uintptr_t>(sB) & 15))) return false;
+  const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  return tiles * 4 >= msb::num_sms();
+}
+
 template <int EPI>
 int launch_fp8(const Fp8Params& p, int grid, cudaStream_t s) {
   auto kern = gemm_fp8_blockscaled_kernel<EPI>;
@@ -296,6 +319,8 @@ MSB_API int msb_gemm_fp8_blockscaled(const void* A, const float* sA_t, const voi
   MSB_REQUIRE(m_tile_group == nullptr || M_total % FBM == 0, "gemm_fp8: grouped rows must be padded to multiples of 128");
   MSB_REQUIRE((fmt_a == 0 || fmt_a == 1) && (fmt_b == 0 || fmt_b == 1), "gemm_fp8: formats must be 0 (e4m3) or 1 (e5m2)");
   MSB_REQUIRE(epilogue >= 0 && epilogue <= 2, "gemm_fp8: bad epilogue %d", epilogue);
+  if (m_tile_group == nullptr && pair_kernel_fits(D, sB, M_total, N, b_scale_rowwise, epilogue, ldd))
+    return msb::gemm2_fp8_blockscaled(A, sA_t, B, sB, D, M_total, N, K, b_scale_rowwise, fmt_a, fmt_b, epilogue, ldd, status, s);
   Fp8Params p;
   memset(&p, 0, sizeof(p));
   int rc = make_tmap_2d(&p.tmA, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)M_total, (uint64_t)K, (uint64_t)K, FBM, FBK);

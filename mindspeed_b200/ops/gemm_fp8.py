@@ -20,9 +20,58 @@ import torch
 
 from . import gemm as G
 from . import loader
+from ._dtypes import code
 from .quant import quant_128x128, quant_1x128
 
 _FMT = {torch.float8_e4m3fn: 0, torch.float8_e5m2: 1}
+_ROW, _COL, _BLOCK = 1, 2, 4
+
+
+def _quant_ok(x, dtype):
+    return (x.is_cuda and loader.lib() is not None and dtype in _FMT and x.dtype in (torch.bfloat16, torch.float16, torch.float32)
+            and x.is_contiguous() and x.data_ptr() % 16 == 0 and x.shape[1] % 128 == 0 and 0 < x.shape[0] < 2 ** 23)
+
+
+def _quant_kernel(x, form, dtype):
+    """One launch of csrc/kernels/quant_fp8.cu: (q, s, qt, st) with None where ``form`` has no such output.  Row and column scales
+    are views of the transposed layout that the GEMM reads."""
+    M, K = x.shape
+    Mp = (M + 127) // 128 * 128
+    new = lambda *shape: torch.empty(*shape, dtype=torch.float32, device=x.device)
+    q = s = qt = st = None
+    if form & (_ROW | _BLOCK):
+        q = torch.empty(M, K, dtype=dtype, device=x.device)
+        s = new(M // 128, K // 128) if form == _BLOCK else new(K // 128, M)
+    if form & (_COL | _BLOCK):
+        qt = torch.empty(K, Mp, dtype=dtype, device=x.device)
+        st = new(K // 128, M // 128) if form == _BLOCK else new(Mp // 128, K)
+    L = loader.require_lib()
+    loader.check(L.msb_quant_fp8(loader.p(x), loader.p(q), loader.p(s), loader.p(qt), loader.p(st), M, K, form, _FMT[dtype], code(x.dtype),
+                                 ctypes.c_void_p(loader.stream_ptr())), "quant_fp8")
+    if form != _BLOCK:
+        s, st = (None if t is None else t.t() for t in (s, st))
+    return q, s, qt, st
+
+
+def quant_activation(x, dtype=torch.float8_e4m3fn, rows=True, cols=False):
+    """x [M, K] -> (q [M, K], s [M, K/128]) and / or, of the transpose padded with zeros to Mp = 128 ceil(M / 128) columns,
+    (qt [K, Mp], st [K, Mp/128]): ``quant_1x128`` of x and of its transpose, from one read of x on a GPU."""
+    if _quant_ok(x, dtype):
+        return _quant_kernel(x, (_ROW if rows else 0) | (_COL if cols else 0), dtype)
+    q = s = qt = st = None
+    if rows:
+        q, s = quant_1x128(x, dtype=dtype)
+    if cols:
+        qt, st = quant_1x128(torch.nn.functional.pad(x, (0, 0, 0, (-x.shape[0]) % 128)).t().contiguous(), dtype=dtype)
+    return q, s, qt, st
+
+
+def quant_weight(w):
+    """w [N, K] -> (q, s [N/128, K/128], qt [K, N], st): ``quant_128x128`` of w and of its transpose (the same tiles, so the same
+    scales and bytes)."""
+    if _quant_ok(w, torch.float8_e4m3fn):
+        return _quant_kernel(w, _BLOCK, torch.float8_e4m3fn)
+    return quant_128x128(w) + quant_128x128(w.t().contiguous())
 
 
 def _ref(xq, xs, wq, ws, w_rowwise, out_dtype):
@@ -118,13 +167,12 @@ class Fp8BlockwiseLinearFn(torch.autograd.Function):
     def forward(ctx, x, w, wcache, grad_dtype):
         x2 = x.reshape(-1, x.shape[-1])
         if wcache is None or "wq" not in wcache:
-            wq, ws = quant_128x128(w.detach())
-            wtq, wts = quant_128x128(w.detach().t().contiguous())
+            wq, ws, wtq, wts = quant_weight(w.detach())
             if wcache is not None:
                 wcache.update(wq=wq, ws=ws, wtq=wtq, wts=wts)
         else:
             wq, ws, wtq, wts = wcache["wq"], wcache["ws"], wcache["wtq"], wcache["wts"]
-        xq, xs = quant_1x128(x2)
+        xq, xs, _, _ = quant_activation(x2)
         y = fp8_gemm(xq, xs, wq, ws, out_dtype=x.dtype if x.dtype in (torch.bfloat16, torch.float32) else torch.bfloat16)
         ctx.save_for_backward(x2, wtq, wts)
         ctx.x_shape, ctx.w_shape, ctx.grad_dtype, ctx.w_dtype = x.shape, w.shape, grad_dtype, w.dtype
@@ -138,17 +186,15 @@ class Fp8BlockwiseLinearFn(torch.autograd.Function):
         M = dy2.shape[0]
         gdt = ctx.grad_dtype or torch.float8_e4m3fn
         dx = dw = None
-        if ctx.needs_input_grad[0]:
-            dyq, dys = quant_1x128(dy2, dtype=gdt)
+        need_dx, need_dw = ctx.needs_input_grad[:2]
+        dyq, dys, dytq, dyts = quant_activation(dy2, gdt, rows=need_dx, cols=need_dw) if need_dx or need_dw else (None,) * 4
+        if need_dx:
             dx = fp8_gemm(dyq, dys, wtq, wts, out_dtype=torch.float32 if dy.dtype == torch.float32 else torch.bfloat16)
             dx = dx.view(ctx.x_shape).to(dy.dtype)
-        if ctx.needs_input_grad[1]:
-            pad = (-M) % 128
-            dyt = torch.nn.functional.pad(dy2, (0, 0, 0, pad)).t().contiguous()      # [N, Mp]
-            xt = torch.nn.functional.pad(x2, (0, 0, 0, pad)).t().contiguous()        # [K, Mp]
-            dytq, dyts = quant_1x128(dyt, dtype=gdt)
-            xtq, xts = quant_1x128(xt)
-            dw = fp8_gemm(dytq, dyts, xtq, xts, out_dtype=torch.float32, w_rowwise=True).to(ctx.w_dtype)
+        if need_dw:
+            _, _, xtq, xts = quant_activation(x2, rows=False, cols=True)
+            dw = fp8_gemm(dytq, dyts, xtq, xts, out_dtype=torch.bfloat16 if ctx.w_dtype == torch.bfloat16 else torch.float32, w_rowwise=True)
+            dw = dw.to(ctx.w_dtype)
         return dx, dw, None, None
 
 

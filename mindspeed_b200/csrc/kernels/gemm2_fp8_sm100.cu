@@ -7,7 +7,7 @@
 // each of 8 warps.  The 128 x 128 single-CTA tile needs twice the shared-memory traffic per product.  Scales of A come from global
 // memory four k-blocks ahead, each slot in its own register; the accumulator is handed back by an arrival of CTA scope, because one
 // of cluster scope waits for those loads (2300 cycles a k-block instead of 1100).  Row-wise scales of B come by TMA and are read as
-// broadcasts.  4096 x 28672 x 4096: block form 809 -> 467 us, weight gradient (row-wise) 2691 -> 840 us.
+// broadcasts.  4096 x 28672 x 4096: block form 809 -> 461 us, weight gradient (row-wise) 2691 -> 769 us.
 //
 // CTA = 12 warps: 0-7 promotion and epilogue (TMEM lane quarter warp & 3, column half warp >> 2: 128 fp32 accumulators per thread),
 // 8 TMA producer, 9 MMA issuer (leader CTA), 10-11 idle (they complete the warpgroup that gives registers away).  Two 256-column

@@ -51,7 +51,7 @@ def test_weight_form_and_special_values(N, K):
     assert torch.equal(torch.nan_to_num(st, nan=-1.0), torch.nan_to_num(quant_1x128(w.t().contiguous())[1], nan=-1.0))
 
 
-@pytest.mark.parametrize("M,N,K", [(2048, 2304, 128), (2500, 1920, 640), (1537, 2944, 256), (256, 9600, 384)])
+@pytest.mark.parametrize("M,N,K", [(2048, 2304, 128), (2500, 1920, 640), (1537, 2944, 256), (256, 9600, 384), (1, 128, 128), (300, 384, 1152)])
 @pytest.mark.parametrize("rowwise", [False, True])
 @pytest.mark.parametrize("out", ["bf16", "f32", "acc"])
 def test_pair_kernel_matches_reference(M, N, K, rowwise, out):

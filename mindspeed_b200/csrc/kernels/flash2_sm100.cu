@@ -275,7 +275,9 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
       const float m_ref = (m_used == -INFINITY) ? 0.f : m_used;
       // probabilities -> packed bf16 over the first 64 columns of S, row sum (masked scores are -inf -> 0)
       const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), nref2 = pack_f32x2(-m_ref, -m_ref);
-      uint64_t sum2[2] = {0ull, 0ull};
+      // the row sum keeps the order of the keys, pair after pair, as the log-sum-exp's last bits always had it; its chain of 64 additions
+      // is shorter than the exponentials of the row
+      float l_tile = 0.f;
 #pragma unroll
       for (int c = 0; c < FB; c += 32) {
         uint32_t pk[16];
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
           unpack_f32x2(fma_f32x2(pack_u32x2(sv[c + 2 * i], sv[c + 2 * i + 1]), scale2, nref2), pa, pb);
           pa = exp2f(pa);
           pb = exp2f(pb);
-          sum2[i & 1] = add_f32x2(sum2[i & 1], pack_f32x2(pa, pb));
+          l_tile += pa + pb;
           pk[i] = pack_bf16(pa, pb);
         }
         tmem_st_32x16(tS + (uint32_t)(c >> 1), pk);
@@ -294,10 +296,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full(t));       // one arrival per warp: 128 on one barrier would serialise
-      float l0, l1, l2, l3;
-      unpack_f32x2(sum2[0], l0, l1);
-      unpack_f32x2(sum2[1], l2, l3);
-      l_run += (l0 + l1) + (l2 + l3);
+      l_run += l_tile;
     }
     // ---- epilogue of this tile ----
     if (n_kv > 0) {

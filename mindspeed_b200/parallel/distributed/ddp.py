@@ -132,7 +132,6 @@ class DistributedDataParallel(nn.Module):
         for p in self.module.parameters():
             if p.requires_grad:
                 p.grad_added_to_main_grad = False
-                p.lookups_in_flight = 0          # embeddings: forward passes of the last step that had no backward don't count
         for buf in self.buffers + self.expert_buffers:
             buf.reset()
 

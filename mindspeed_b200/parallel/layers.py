@@ -353,31 +353,53 @@ class VocabUtility:
         return VocabUtility.vocab_range_from_per_partition_vocab_size(divide(global_vocab, world_size), rank, world_size)
 
 
+class _Lookup:
+    """A lookup of ``weight`` whose backward has not run.  It ends with its backward, or with the graph that it belongs to: a forward
+    pass that is never differentiated, or one that checkpointing runs again only for its saved tensors, does not stay open."""
+    __slots__ = ("weight", "open")
+    lock = threading.RLock()              # a graph may be freed, and its lookups close, while this thread is in here
+
+    def __init__(self, weight):
+        self.weight, self.open = weight, True
+        with _Lookup.lock:
+            weight.lookups_in_flight = getattr(weight, "lookups_in_flight", 0) + 1
+
+    def close(self) -> int:
+        """Ends this lookup; how many others of the table are open."""
+        with _Lookup.lock:
+            if self.open:
+                self.open = False
+                self.weight.lookups_in_flight -= 1
+            return self.weight.lookups_in_flight
+
+    def __del__(self):
+        self.close()
+
+
 class _EmbeddingFn(torch.autograd.Function):
     """Embedding lookup whose gradient rows are added straight into the fp32 ``weight.main_grad`` (the accumulation fusion of the
     linear layers: no dense gradient, the data-parallel wrapper is told through ``weight._main_grad_ready_cb``).  A table may be
     looked up several times before backward (multi-token prediction): the wrapper is told once no lookup is outstanding, and starts
-    a bucket it was never told about when it finishes the step."""
-    lock = threading.Lock()
+    a bucket it was never told about when it finishes the step.
+
+    The parameter is kept as it is, not among the saved tensors: what saved-tensor hooks (host swap, checkpointing) hand back is
+    another tensor, without the accumulator, and the gradient does not depend on the weight's values."""
 
     @staticmethod
     def forward(ctx, ids, weight):
-        ctx.save_for_backward(ids, weight)
-        with _EmbeddingFn.lock:
-            weight.lookups_in_flight = getattr(weight, "lookups_in_flight", 0) + 1
+        ctx.save_for_backward(ids)
+        ctx.lookup = _Lookup(weight)
         return F.embedding(ids, weight)
 
     @staticmethod
     def backward(ctx, dout):
         from ..ops.permute import add_rows_
-        ids, weight = ctx.saved_tensors
+        ids, = ctx.saved_tensors
+        weight = ctx.lookup.weight
         add_rows_(weight.main_grad, ids.reshape(-1).long().contiguous(), dout.reshape(-1, dout.shape[-1]).contiguous())
         weight.grad_added_to_main_grad = True
-        with _EmbeddingFn.lock:
-            weight.lookups_in_flight -= 1
-            last = weight.lookups_in_flight <= 0
         cb = getattr(weight, "_main_grad_ready_cb", None)
-        if cb is not None and last:
+        if ctx.lookup.close() <= 0 and cb is not None:
             cb(weight)
         return None, None
 

@@ -69,6 +69,7 @@ class GPTModel(nn.Module):
                 self.output_layer.weight.shared_embedding = True
         if pre_process and share_embeddings_and_output_weights:
             self.embedding.word_embeddings.weight.shared_embedding = True
+            self.embedding.word_embeddings.weight.zero_out_wgrad = True       # looked up here as well: complete after the lookup's backward
         self.mtp = None
         if getattr(config, "mtp_num_layers", None) and post_process:
             from .mtp import MultiTokenPredictionBlock

@@ -94,13 +94,16 @@ class DistributedDataParallel(nn.Module):
         return self.module(*a, **k)
 
     def _on_main_grad_ready(self, p):
+        if getattr(p, "zero_out_wgrad", False):
+            return                     # the lookup's share of a shared table is still to come, through autograd and the hook
         self._param_to_buffer[id(p)].register_grad_ready(p)
 
     def _make_hook(self, p):
         def hook(param):
+            # a fused op adds to main_grad by itself and hands autograd nothing: what autograd has is another use's share (the lookup of
+            # a table that the output layer shares, a penalty on the weights)
             if param.grad is not None:
-                if not getattr(param, "grad_added_to_main_grad", False):
-                    param.main_grad.add_(param.grad.to(param.main_grad.dtype))
+                param.main_grad.add_(param.grad.to(param.main_grad.dtype))
                 param.grad = None
             self._param_to_buffer[id(param)].register_grad_ready(param)
         return hook

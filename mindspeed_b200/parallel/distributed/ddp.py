@@ -106,6 +106,7 @@ class DistributedDataParallel(nn.Module):
                 param.main_grad.add_(param.grad.to(param.main_grad.dtype))
                 param.grad = None
             self._param_to_buffer[id(param)].register_grad_ready(param)
+        hook.fills_main_grad = True
         return hook
 
     @contextlib.contextmanager

@@ -444,13 +444,15 @@ class VocabParallelEmbedding(nn.Module):
 
     def _fused(self, ids):
         """Whether the gradient goes straight into ``main_grad``: not for a weight that the output layer shares (its two gradients
-        meet in autograd), nor where the sums have to come out the same in every run."""
+        meet in the wrapper's hook), nor where the sums have to come out the same in every run, or somebody has hooked the weight's
+        gradient."""
         w = self.weight
         main = getattr(w, "main_grad", None)
         return (self.fuse_grad and w.is_cuda and w.requires_grad and torch.is_grad_enabled() and not self.deterministic_mode
                 and not torch.are_deterministic_algorithms_enabled() and not getattr(w, "shared_embedding", False)
                 and torch.is_tensor(main) and main.dtype == torch.float32 and main.is_contiguous() and main.shape == w.shape
-                and w.dtype in (torch.bfloat16, torch.float16, torch.float32) and ids.numel() > 0)
+                and w.dtype in (torch.bfloat16, torch.float16, torch.float32) and ids.numel() > 0
+                and not w._backward_hooks and all(getattr(h, "fills_main_grad", False) for h in (w._post_accumulate_grad_hooks or {}).values()))
 
     def sharded_state_dict(self, prefix="", sharded_offsets=(), metadata=None):
         from ..checkpointing.sharded import make_tp_sharded_tensors

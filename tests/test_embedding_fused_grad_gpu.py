@@ -43,3 +43,26 @@ def test_shared_tables_and_missing_accumulators_keep_the_dense_gradient():
     del m.weight.main_grad
     m(torch.tensor([[1, 1, 3]], device="cuda")).sum().backward()
     assert m.weight.grad[3, 0].item() == 1
+
+
+def test_hooked_weights_keep_the_dense_gradient():
+    ids = torch.tensor([[1, 1, 3]], device="cuda")
+    for register in ("register_hook", "register_post_accumulate_grad_hook"):
+        m, seen = _table(10, 16), []
+        handle = getattr(m.weight, register)(lambda t: seen.append(tuple(t.shape)))
+        m(ids).sum().backward()
+        assert seen == [(10, 16)] and m.weight.grad[1, 0].item() == 2 and not m.told
+        handle.remove()
+        m.weight.grad = None
+        m(ids).sum().backward()
+        assert len(seen) == 1 and m.weight.grad is None and m.weight.main_grad[1, 0].item() == 2
+
+
+def test_the_wrappers_own_hook_does_not_count():
+    def hook(p):
+        assert p.grad is None                         # the node runs, but autograd has no gradient for this weight
+    hook.fills_main_grad = True
+    m = _table(10, 16)
+    m.weight.register_post_accumulate_grad_hook(hook)
+    m(torch.tensor([[1, 1, 3]], device="cuda")).sum().backward()
+    assert m.weight.grad is None and m.weight.main_grad[3, 0].item() == 1 and len(m.told) == 1

@@ -21,6 +21,7 @@ from ..parallel import parallel_state as ps
 from ..parallel.layers import ColumnParallelLinear, RowParallelLinear, divide, linear_classes
 from ..parallel.random import get_cuda_rng_tracker
 from .norms import build_norm
+from .observed import observed
 
 
 class _PackedRope(torch.autograd.Function):
@@ -122,6 +123,8 @@ class CoreAttention(nn.Module):
             out = attn_ops.flash_attention(q, k, v, causal=self.causal, softmax_scale=self.softmax_scale, backend=backend)
         return self._finish(out)
 
+    own_forward = forward          # models/observed.py
+
     def _finish(self, out):
         if self.dropout_p > 0 and self.training:
             with get_cuda_rng_tracker().fork():
@@ -133,12 +136,11 @@ class CoreAttention(nn.Module):
         """The attention of a packed QKV activation without taking it apart, or None where ``forward`` would not run the plain
         self-attention of the hand-written kernels (or where somebody has hooked or replaced it)."""
         cfg = self.config
-        if (type(self) is not CoreAttention or "forward" in self.__dict__ or self._forward_hooks or self._forward_pre_hooks
-                or self._backward_hooks or self._backward_pre_hooks):
+        if observed(self, CoreAttention) or attn_ops.flash_attention is not attn_ops.OWN_FLASH_ATTENTION:
             return None
         if (cfg.optimization_level < 1 or getattr(cfg, "attention_backend", "auto") not in ("auto", "sm100") or self.alibi_slopes is not None
                 or packed_seq_params is not None or (attention_mask is not None and not self.causal)
-                or ps.get_context_parallel_world_size() > 1 or self._window(qkv.shape[0], qkv.shape[0]) is not None or not qkv.is_cuda):
+                or ps.get_context_parallel_world_size() > 1 or self._window(qkv.shape[0], qkv.shape[0]) is not None):
             return None
         from ..ops.flash_sm100_impl import flash_attention_packed, packed_supports
         if not packed_supports(qkv, groups, qpg):

@@ -92,6 +92,10 @@ def flash_attention(q, k, v, causal=True, softmax_scale=None, return_lse=False, 
     return attention_ref(q, k, v, causal, softmax_scale, return_lse=return_lse)
 
 
+#: to tell whether a program has put its own attention in the place of ``flash_attention`` (paths that pass it by ask)
+OWN_FLASH_ATTENTION = flash_attention
+
+
 # ---------------------------------------------------------------------------------------------------------
 # Block primitives for ring / KV-allgather attention: forward returning LSE, backward taking the GLOBAL output
 # and LSE (so partial blocks of one softmax row can be differentiated independently).

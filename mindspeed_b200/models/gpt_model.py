@@ -15,6 +15,7 @@ from ..parallel import parallel_state as ps
 from ..parallel.cross_entropy import vocab_parallel_cross_entropy
 from ..parallel.layers import ColumnParallelLinear
 from .embedding import LanguageModelEmbedding
+from .observed import observed
 from .rotary import RotaryEmbedding, cp_local_positions
 from .transformer import TransformerBlock
 
@@ -128,7 +129,8 @@ class GPTModel(nn.Module):
         mtp_loss = None
         if self.mtp is not None and labels is not None and self.training:
             mtp_loss = self.mtp(hidden, input_ids, position_ids, labels, loss_mask, self, rpe, attention_mask)
-        if labels is None and hidden.shape[1] > 1 and ps.get_tensor_model_parallel_world_size() == 1:
+        if (labels is None and hidden.shape[1] > 1 and ps.get_tensor_model_parallel_world_size() == 1
+                and not observed(self.output_layer, ColumnParallelLinear)):      # who watches it sees [s, b, h] always
             # sample-major logits: the hidden states change places before the product, not the (vocabulary / hidden times larger) logits
             logits, _ = self.output_layer(hidden.transpose(0, 1).contiguous(), weight=weight)
             return logits

@@ -278,6 +278,8 @@ class ColumnParallelLinear(nn.Module):
             y = M.gather_from_tensor_model_parallel_region(y, self.tp_group)
         return y, (self.bias if self.skip_bias_add else None)
 
+    own_forward = forward          # models/observed.py
+
     def sharded_state_dict(self, prefix="", sharded_offsets=(), metadata=None):
         from ..checkpointing.sharded import make_tp_sharded_tensors
         return make_tp_sharded_tensors(self.state_dict(prefix="", keep_vars=True), prefix, {"weight": 0, "bias": 0},

@@ -1,6 +1,6 @@
 // Routing tables of a mixture-of-experts layer from its routing map, without the host knowing any count: the rows of the dispatched
 // activation ordered by expert and, inside an expert, by token.
-//   count   counts[e] = tokens routed to e
+//   count   tokens routed to e
 //   place   rows of e start at the sum of the counts before e: idx[r] = token, row_prob[r] = probs[token, e]
 //   scatter (backward) dprobs[idx[r], e] = g[r], zero elsewhere
 // A block per expert walks its column of the map.  Bound by launches (the map is T x E bytes); it stands in for two transposes, two
@@ -39,13 +39,21 @@ __device__ __forceinline__ long long first_row(const long long* counts, int e, l
   return *sh;
 }
 
+// counts[e]: found[e], cut where the caller's rows end, so that what reads the rows by these counts stays inside them; a map whose entries
+// are not as many as the caller said leaves a code in the status word.
 template <typename T>
-__global__ void __launch_bounds__(RT) route_place_kernel(const uint8_t* __restrict__ map, const T* __restrict__ probs, const long long* __restrict__ counts,
-                                                         long long* __restrict__ idx, T* __restrict__ row_prob, long long tokens, int E, long long rows) {
+__global__ void __launch_bounds__(RT) route_place_kernel(const uint8_t* __restrict__ map, const T* __restrict__ probs, const long long* __restrict__ found,
+                                                         long long* __restrict__ counts, long long* __restrict__ idx, T* __restrict__ row_prob,
+                                                         long long tokens, int E, long long rows, unsigned int* status) {
   __shared__ long long base_sh;
   __shared__ int warp_n[RT / 32];
   const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  long long base = first_row(counts, e, &base_sh);
+  long long base = first_row(found, e, &base_sh);
+  if (threadIdx.x == 0) {
+    const long long end = base + found[e];
+    counts[e] = max(min(end, rows) - base, 0ll);
+    if (e == E - 1 && end != rows) atomicCAS(status, 0u, 0x702u);
+  }
   for (long long t0 = 0; t0 < tokens; t0 += RT) {
     const long long t = t0 + threadIdx.x;
     const bool on = t < tokens && map[t * E + e] != 0;
@@ -76,13 +84,15 @@ __global__ void route_scatter_kernel(const T* __restrict__ g, const long long* _
 }
 }  // namespace
 
-// map [tokens, E] bytes, probs [tokens, E]; counts [E], idx [rows], row_prob [rows].  rows: the number of non-zero bytes of the map.
-MSB_API int msb_moe_route(const void* map, const void* probs, long long* counts, long long* idx, void* row_prob, long long tokens, int E,
-                          long long rows, int dtype, cudaStream_t s) {
+// map [tokens, E] bytes, probs [tokens, E]; counts [E], idx [rows], row_prob [rows]; found: scratch [E].  rows: the number of non-zero bytes
+// of the map.
+MSB_API int msb_moe_route(const void* map, const void* probs, long long* found, long long* counts, long long* idx, void* row_prob, long long tokens,
+                          int E, long long rows, int dtype, unsigned int* status, cudaStream_t s) {
   MSB_REQUIRE(E > 0 && tokens > 0 && rows >= 0, "moe_route: bad shape tokens=%lld E=%d rows=%lld", tokens, E, rows);
-  route_count_kernel<<<E, RT, 0, s>>>((const uint8_t*)map, counts, tokens, E);
+  MSB_REQUIRE(status != nullptr, "moe_route: status word is required");
+  route_count_kernel<<<E, RT, 0, s>>>((const uint8_t*)map, found, tokens, E);
   MSB_CHECK_LAUNCH("moe_route_count");
-  MSB_DISPATCH_FLOAT(dtype, T, route_place_kernel<T><<<E, RT, 0, s>>>((const uint8_t*)map, (const T*)probs, counts, idx, (T*)row_prob, tokens, E, rows));
+  MSB_DISPATCH_FLOAT(dtype, T, route_place_kernel<T><<<E, RT, 0, s>>>((const uint8_t*)map, (const T*)probs, found, counts, idx, (T*)row_prob, tokens, E, rows, status));
   MSB_CHECK_LAUNCH("moe_route_place");
   return 0;
 }

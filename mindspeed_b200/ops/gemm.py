@@ -17,6 +17,10 @@ EPI_BF16, EPI_F32, EPI_F32_ACC = 0, 1, 2
 _status = {}
 
 
+#: codes of the status word that are not expired waits
+_MEANING = {0x702: "a routing map with another number of entries than stated"}
+
+
 def status_word(device) -> torch.Tensor:
     """Per-device error word written by a kernel whose bounded wait expired (0 = healthy)."""
     t = _status.get(device)
@@ -27,14 +31,14 @@ def status_word(device) -> torch.Tensor:
 
 
 def check_status(device=None):
-    """Synchronising check; raises if any GEMM-class kernel recorded a time-out since the last check."""
+    """Synchronising check; raises if any kernel recorded a time-out, or one of ``_MEANING``, since the last check."""
     for dev, t in _status.items():
         if device is not None and dev != device:
             continue
         v = int(t[0].item())
         if v != 0:
             t.zero_()
-            raise RuntimeError(f"sm_100a kernel reported a bounded-wait time-out, code 0x{v:x} on {dev}")
+            raise RuntimeError(f"sm_100a kernel reported {_MEANING.get(v, 'a bounded-wait time-out')}, code 0x{v:x} on {dev}")
 
 
 class cta_limit:

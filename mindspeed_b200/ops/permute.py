@@ -5,6 +5,7 @@ import ctypes
 
 import torch
 
+from . import gemm as G
 from . import loader
 from ._dtypes import CODE, code
 
@@ -83,12 +84,12 @@ class _RouteTables(torch.autograd.Function):
         L = loader.require_lib()
         T, E = routing_map.shape
         probs = probs.contiguous()
-        counts = torch.empty(E, dtype=torch.int64, device=probs.device)
+        found, counts = (torch.empty(E, dtype=torch.int64, device=probs.device) for _ in range(2))
         idx = torch.zeros(rows, dtype=torch.int64, device=probs.device)
         row_prob = torch.zeros(rows, dtype=probs.dtype, device=probs.device)
-        loader.check(L.msb_moe_route(loader.p(routing_map.contiguous()), loader.p(probs), loader.p(counts), loader.p(idx), loader.p(row_prob),
-                                     ctypes.c_longlong(T), E, ctypes.c_longlong(rows), code(probs.dtype),
-                                     ctypes.c_void_p(loader.stream_ptr())), "moe_route")
+        loader.check(L.msb_moe_route(loader.p(routing_map.contiguous()), loader.p(probs), loader.p(found), loader.p(counts), loader.p(idx),
+                                     loader.p(row_prob), ctypes.c_longlong(T), E, ctypes.c_longlong(rows), code(probs.dtype),
+                                     loader.p(G.status_word(probs.device)), ctypes.c_void_p(loader.stream_ptr())), "moe_route")
         ctx.save_for_backward(idx, counts)
         ctx.shape = (T, E)
         ctx.mark_non_differentiable(idx, counts)
@@ -113,5 +114,6 @@ def route_supports(probs, routing_map) -> bool:
 
 def route_tables(probs, routing_map, rows):
     """probs / routing_map [T, E], ``rows`` = number of entries of the map -> (token of every dispatched row, expert after expert and
-    inside an expert by token [rows]; its probability [rows], differentiable; rows per expert [E]), all on the device."""
+    inside an expert by token [rows]; its probability [rows], differentiable; rows per expert [E]), all on the device.  Where the map has
+    another number of entries, what does not fit is left out and ``ops.gemm.check_status`` raises."""
     return _RouteTables.apply(probs, routing_map, rows)

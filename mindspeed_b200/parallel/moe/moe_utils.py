@@ -44,6 +44,20 @@ def unpermute(permuted_tokens, sorted_indices, restore_shape, probs=None, routin
     return out
 
 
+def mark_rows_per_token(routing_map, n: int):
+    """Notes on a routing map that every token has exactly ``n`` entries.  The note holds for the values that the map has now."""
+    routing_map.rows_per_token = (n, None if routing_map.is_inference() else routing_map._version)
+
+
+def rows_per_token(routing_map) -> Optional[int]:
+    """What ``mark_rows_per_token`` noted, or None when there is no note, the map has been written to since, or (inference tensors count
+    no versions) nobody could tell."""
+    note = getattr(routing_map, "rows_per_token", None)
+    if note is None or routing_map.is_inference() or note[1] != routing_map._version:
+        return None
+    return note[0]
+
+
 def sort_chunks_by_idxs(x, split_sizes, sorted_idxs, probs=None):
     """Split ``x`` along dim 0 into chunks of ``split_sizes`` and concatenate them in ``sorted_idxs`` order
     (reference Triton version: mindspeed/ops/triton/sort_chunks_by_idx.py:24,119)."""

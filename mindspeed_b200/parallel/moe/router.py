@@ -6,7 +6,7 @@ import torch
 import torch.nn as nn
 
 from .. import parallel_state as ps
-from .moe_utils import (MoEAuxLossAutoScaler, sequence_load_balancing_loss_func, switch_load_balancing_loss_func,
+from .moe_utils import (MoEAuxLossAutoScaler, mark_rows_per_token, sequence_load_balancing_loss_func, switch_load_balancing_loss_func,
                         topk_softmax_with_capacity, track_moe_metrics, z_loss_func)
 
 
@@ -103,7 +103,7 @@ class TopKRouter(nn.Module):
             scores_for_loss = sg / (sg.sum(-1, keepdim=True) + 1e-20)
         probs = self._aux(scores_for_loss, rmap, tpe, probs, seq_shape)
         if cfg.moe_expert_capacity_factor is None:
-            rmap.rows_per_token = self.topk          # no token was dropped: the dispatcher knows its row count without asking the device
+            mark_rows_per_token(rmap, self.topk)     # no token was dropped: the dispatcher knows its row count without asking the device
         return probs, rmap
 
     def update_expert_bias(self):

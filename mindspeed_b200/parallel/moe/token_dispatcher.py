@@ -19,7 +19,7 @@ import torch.distributed as dist
 
 from .. import mappings as M
 from .. import parallel_state as ps
-from .moe_utils import permute, sort_chunks_by_idxs, unpermute
+from .moe_utils import permute, rows_per_token, sort_chunks_by_idxs, unpermute
 
 
 class MoETokenDispatcher:
@@ -151,7 +151,7 @@ class MoEAlltoAllTokenDispatcher(MoETokenDispatcher):
         h = hidden.reshape(-1, hidden.shape[-1])
         self.routing_map, self.probs = routing_map, probs
         self.restore_shape = h.shape
-        per_token = getattr(routing_map, "rows_per_token", None)
+        per_token = rows_per_token(routing_map)
         if per_token is not None and self.ep_size == 1 and self.fused_permute:
             from ...ops.permute import gather_rows, route_supports, route_tables
             if route_supports(probs, routing_map):

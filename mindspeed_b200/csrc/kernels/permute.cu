@@ -113,12 +113,16 @@ __global__ void sum_chains_kernel(const T* __restrict__ src, const float* __rest
 }
 // out[idx[r]] += src[r] in fp32, for tables that are far larger than the rows that touch them (gradient of an embedding into its
 // accumulator): no dense gradient is formed, cleared, widened and added.  Rows may repeat often, so the sums are atomics, four
-// columns each: 8192 rows of 4096 add in 74 us; forming, widening and adding the dense gradient of a 32000-row table took 1.1 ms.
+// columns each: 8192 rows of 4096 add in 74 us; forming, widening and adding the dense gradient of a 32000-row table took 1.1 ms.  Rows
+// with a negative index are not read: under a vocabulary split most ids belong to other ranks, and their zeros added to one row would
+// queue at its addresses.
 template <typename T>
 __global__ void add_rows_kernel(const T* __restrict__ src, const long long* __restrict__ idx, float* __restrict__ out, long long n, int cols, int vec) {
   for (long long r = blockIdx.x; r < n; r += gridDim.x) {
+    const long long o = idx[r];
+    if (o < 0) continue;
     const T* s = src + r * (long long)cols;
-    float* d = out + idx[r] * (long long)cols;
+    float* d = out + o * (long long)cols;
     if (vec) {
       for (int c = threadIdx.x * 8; c < cols; c += blockDim.x * 8) {
         Vec8<T> t;
@@ -163,7 +167,7 @@ MSB_API int msb_scatter_add_rows(const void* src, const long long* idx, const fl
   MSB_CHECK_LAUNCH("scatter_add_rows");
   return 0;
 }
-// out [rows, cols] fp32: out[idx[r]] += src[r] for r < n.
+// out [rows, cols] fp32: out[idx[r]] += src[r] for r < n with idx[r] >= 0.
 MSB_API int msb_add_rows_f32(const void* src, const long long* idx, float* out, long long n, int cols, int dtype, cudaStream_t s) {
   if (n == 0 || cols == 0) return 0;
   const int vec = (cols % 8 == 0 && (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(out)) % 16 == 0) ? 1 : 0;

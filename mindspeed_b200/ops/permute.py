@@ -71,7 +71,7 @@ def scatter_add_rows(src, idx, rows, weight=None):
 
 
 def add_rows_(out, idx, src):
-    """out[idx[r]] += src[r]; ``out`` fp32 contiguous [rows, cols], rows may repeat (sums in no fixed order)."""
+    """out[idx[r]] += src[r] where idx[r] >= 0; ``out`` fp32 contiguous [rows, cols], rows may repeat (sums in no fixed order)."""
     L = loader.require_lib()
     loader.check(L.msb_add_rows_f32(loader.p(src), loader.p(idx), loader.p(out), ctypes.c_longlong(idx.numel()), src.shape[1],
                                     code(src.dtype), ctypes.c_void_p(loader.stream_ptr())), "add_rows_f32")

@@ -388,8 +388,9 @@ class _EmbeddingFn(torch.autograd.Function):
     another tensor, without the accumulator, and the gradient does not depend on the weight's values."""
 
     @staticmethod
-    def forward(ctx, ids, weight):
-        ctx.save_for_backward(ids)
+    def forward(ctx, ids, weight, elsewhere):
+        """``elsewhere`` (bool, or None): ids of other ranks, looked up as row 0 and masked afterwards; they have no gradient."""
+        ctx.save_for_backward(ids if elsewhere is None else ids.masked_fill(elsewhere, -1))
         ctx.lookup = _Lookup(weight)
         return F.embedding(ids, weight)
 
@@ -403,7 +404,7 @@ class _EmbeddingFn(torch.autograd.Function):
         cb = getattr(weight, "_main_grad_ready_cb", None)
         if ctx.lookup.close() <= 0 and cb is not None:
             cb(weight)
-        return None, None
+        return None, None, None
 
 
 class VocabParallelEmbedding(nn.Module):
@@ -435,8 +436,8 @@ class VocabParallelEmbedding(nn.Module):
             mask = (input_ < self.vocab_start_index) | (input_ >= self.vocab_end_index)
             masked = (input_ - self.vocab_start_index).masked_fill(mask, 0)
         else:
-            masked = input_
-        out = _EmbeddingFn.apply(masked, self.weight) if self._fused(masked) else F.embedding(masked, self.weight)
+            mask, masked = None, input_
+        out = _EmbeddingFn.apply(masked, self.weight, mask) if self._fused(masked) else F.embedding(masked, self.weight)
         if self.world > 1:
             out = out.masked_fill(mask.unsqueeze(-1), 0.0)
         if self.reduce_scatter_embeddings:

@@ -64,3 +64,15 @@ def test_add_rows_into_fp32_table(n, rows, cols, dtype):
     size = out.double().abs().index_add(0, idx, src.double().abs())
     add_rows_(out, idx, src)
     assert ((out.double() - want).abs() <= (n + 1) * 2.0 ** -24 * size).all()
+
+
+def test_add_rows_leaves_out_negative_rows():
+    """Neither read (a NaN there would show) nor added."""
+    from mindspeed_b200.ops.permute import add_rows_
+    src = torch.full((40, 16), float("nan"), device="cuda")
+    idx = torch.full((40,), -1, device="cuda")
+    idx[5], idx[9] = 2, 0
+    src[5], src[9] = 1.0, 2.0
+    out = torch.zeros(3, 16, device="cuda")
+    add_rows_(out, idx, src)
+    assert out[:, 0].tolist() == [2.0, 0.0, 1.0] and not out.isnan().any()

@@ -63,3 +63,20 @@ def test_a_graph_that_is_dropped_closes_its_lookups(table):
     table(torch.tensor([4]))                                   # never differentiated
     kept.sum().backward()
     assert len(table.told) == 1 and table.weight.lookups_in_flight == 0
+
+
+def test_ids_of_other_ranks_add_nothing(table, monkeypatch):
+    """A vocabulary split: rows 20 .. 39 of 60 are here. Every other id is left out of the sum instead of adding zeros to row 0."""
+    from mindspeed_b200.ops import permute
+    from mindspeed_b200.parallel import mappings as M
+    table.world, table.vocab_start_index, table.vocab_end_index = 3, 20, 40
+    monkeypatch.setattr(M, "reduce_from_tensor_model_parallel_region", lambda x, group=None: x)
+    seen = []
+    monkeypatch.setattr(permute, "add_rows_", lambda out, idx, src: (seen.append(idx), out.index_add_(0, idx[idx >= 0], src[idx >= 0]))[1])
+    ids = torch.tensor([[0, 19, 20, 39], [40, 59, 25, 25]])
+    out = table(ids)
+    here = torch.tensor([[0, 0, 1, 1], [0, 0, 1, 1]], dtype=torch.bool)
+    assert torch.equal(out[here], table.weight.detach()[ids[here] - 20]) and not out[~here].any()
+    out.backward(torch.ones_like(out))
+    assert seen[0].tolist() == [-1, -1, 0, 19, -1, -1, 5, 5]
+    assert table.weight.main_grad[:, 0].tolist() == [1.0 if r in (0, 19) else 2.0 if r == 5 else 0.0 for r in range(20)]

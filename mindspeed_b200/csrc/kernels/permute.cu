@@ -1,8 +1,10 @@
 // MoE token permutation: row gather and (optionally weighted) row scatter-add with fp32 accumulation.
-// The scatter-add runs as a gather: every source row enters its output row's table of eight slots, or a list behind it, then a block
-// per output row sums them in registers (slots in ascending order, so that up to eight the order in which threads run does not
-// show) and writes the result once.  Bound by the read of the source rows.  (As fp32 atomics into a zeroed buffer that
-// was rounded afterwards, 24576 rows of 4096 took 180 us beside 25 us for the passes around it.)
+// The scatter-add runs as a gather: every source row enters its output row's table of eight slots, then a block per output row sums
+// them in registers (in ascending order, so that up to eight the order in which threads run does not show) and writes the result
+// once.  Bound by the read of the source rows.  (As fp32 atomics into a zeroed buffer that was rounded afterwards, 24576 rows of 4096
+// took 180 us beside 25 us for the passes around it.)  Source rows behind the slots, which a token of a mixture of experts has not but a
+// repeated index has, are listed output row by output row and summed in pieces of 32, a block each; only where an output row has
+// several pieces do these meet in atomics.
 // reference semantics: npu_moe_token_permute / npu_moe_token_unpermute
 // (mindspeed/ops/csrc/cann/npu_moe_token_permute.cpp, npu_moe_token_unpermute.cpp).
 #include "msb_common.cuh"
@@ -23,93 +25,229 @@ __global__ void gather_rows_kernel(const T* __restrict__ x, const long long* __r
     }
   }
 }
-constexpr int SLOTS = 8;               // source rows of an output row that are found without walking a list (a token's experts)
-constexpr int CHAIN = 64;              // list entries taken at a time (and put in ascending order)
+constexpr int SLOTS = 8;               // source rows of an output row that need no list (a token's experts)
+constexpr int PIECE = 32;              // source rows behind the slots that a block sums
 
-// scratch of one call, long long each: count [rows] | head of the overflow list [rows] | slots [rows, 8] | next [n]
-struct Chains {
-  long long *count, *head, *slot, *next;
-  __host__ __device__ Chains(long long* p, long long rows) : count(p), head(p + rows), slot(p + 2 * rows), next(p + (2 + SLOTS) * rows) {}
-};
-
-__global__ void chain_rows_kernel(const long long* __restrict__ idx, Chains c, long long n) {
-  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {
-    const long long o = idx[r], pos = (long long)atomicAdd(reinterpret_cast<unsigned long long*>(c.count + o), 1ull);
-    if (pos < SLOTS) c.slot[o * SLOTS + pos] = r;
-    else c.next[r] = (long long)atomicExch(reinterpret_cast<unsigned long long*>(c.head + o), (unsigned long long)r);
+// Scratch of one call, long long each.  An output row is full when it has more than SLOTS source rows; F = most full rows there can be.
+struct Tables {
+  long long *count;                    // [rows] source rows of an output row
+  long long *ticket, *n_full, *n_task; // blocks that have placed their rows; full rows; pieces.  count and these are cleared first
+  long long *full_of;                  // [rows] number of an output row among the full ones
+  long long *slot;                     // [rows, SLOTS]
+  long long *row, *off, *done;         // [F] of a full row: its output row, where its list starts, pieces that are summed
+  long long *pos, *list;               // [n] place of a source row in its output row; the lists behind the slots
+  long long *task;                     // [2 (n / PIECE + F)] full row and number of a piece
+  static long long most_full(long long n, long long rows) { return rows < n / (SLOTS + 1) ? rows : n / (SLOTS + 1); }
+  static long long most_tasks(long long n, long long rows) { return n / PIECE + most_full(n, rows); }
+  Tables(long long* p, long long n, long long rows) {
+    const long long f = most_full(n, rows);
+    auto take = [&p](long long k) { long long* at = p; p += k; return at; };
+    count = take(rows); ticket = take(1); n_full = take(1); n_task = take(1);
+    full_of = take(rows); slot = take(rows * SLOTS);
+    row = take(f); off = take(f); done = take(f);
+    pos = take(n); list = take(n); task = take(2 * most_tasks(n, rows));
   }
+};
+__device__ __forceinline__ long long fetch_add(long long* p, long long v) {
+  return (long long)atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v);
 }
 
-// weight (optional): one factor per source row
-template <typename T>
-__global__ void sum_chains_kernel(const T* __restrict__ src, const float* __restrict__ weight, Chains ch, T* __restrict__ out, long long rows,
-                                  int cols, int vec) {
-  __shared__ long long list[CHAIN];
-  __shared__ int count;
-  for (long long o = blockIdx.x; o < rows; o += gridDim.x) {
-    T* dst = out + (size_t)o * cols;
-    const long long n = ch.count[o];
-    // columns in chunks of 8 per thread; rows with more source rows than a list holds take several rounds per chunk
-    for (int c0 = 0; c0 < cols; c0 += (int)blockDim.x * 8) {
-      const int c = c0 + (int)threadIdx.x * 8;
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      long long at = n > SLOTS ? ch.head[o] : -1;      // overflow that is still to come
-      bool first = true;
-      do {
-        __syncthreads();
-        if (first) {                                   // the slots, every one ranked by its own thread
-          const int k = (int)(n < SLOTS ? n : SLOTS);
-          if ((int)threadIdx.x < k) {
-            const long long mine = ch.slot[o * SLOTS + threadIdx.x];
-            int rank = 0;
-            for (int i = 0; i < k; ++i) rank += ch.slot[o * SLOTS + i] < mine ? 1 : 0;
-            list[rank] = mine;
-          }
-          if (threadIdx.x == 0) count = k;
-        } else if (threadIdx.x == 0) {
-          int k = 0;
-          for (long long w = at; k < CHAIN && w >= 0; ++k, w = ch.next[w]) {
-            int j = k;
-            for (; j > 0 && list[j - 1] > w; --j) list[j] = list[j - 1];
-            list[j] = w;
-          }
-          count = k;
-        }
-        __syncthreads();
-        const int k = count;
-        if (!first) {                                  // everyone moves on to what the next round takes
-          if (k == CHAIN) { for (int i = 0; i < CHAIN; ++i) at = ch.next[at]; }
-          else at = -1;
-        }
-        first = false;
-#pragma unroll 4
-        for (int i = 0; i < k; ++i) {
-          const long long r = list[i];
-          const float w = weight ? weight[r] : 1.f;
-          const T* s = src + (size_t)r * cols;
-          if (vec) {
-            if (c < cols) {
-              Vec8<T> t;
-              float f[8];
-              t.load(s + c);
-              t.to_float(f);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) acc[j] = fmaf(f[j], w, acc[j]);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) if (c + j < cols) acc[j] = fmaf(to_f(s[c + j]), w, acc[j]);
-          }
-        }
-      } while (at >= 0);
-      if (vec) {
-        if (c < cols) { Vec8<T> t; t.from_float(acc); t.store(dst + c); }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) if (c + j < cols) dst[c + j] = from_f<T>(acc[j]);
+// Places of the source rows.  Lanes of a warp with the same output row count once together.  The last block to finish deals the lists'
+// ranges and the pieces to the full rows.
+__global__ void __launch_bounds__(1024) place_rows_kernel(const long long* __restrict__ idx, Tables t, long long n) {
+  __shared__ bool last;
+  __shared__ unsigned long long next_off, next_task;
+  const int lane = threadIdx.x & 31;
+  // all lanes of a warp take part in every round
+  for (long long r0 = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); r0 < n; r0 += (long long)gridDim.x * blockDim.x) {
+    const long long r = r0 + lane, o = r < n ? idx[r] : -1;
+    const unsigned int same = __match_any_sync(0xffffffffu, (unsigned long long)o);
+    const int leader = __ffs(same) - 1;
+    long long pos = 0;
+    if (lane == leader && r < n) pos = fetch_add(t.count + o, __popc(same));
+    pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(same & ((1u << lane) - 1u));
+    if (r < n) {
+      t.pos[r] = pos;
+      if (pos < SLOTS) t.slot[o * SLOTS + pos] = r;
+      if (pos == SLOTS) {
+        const long long f = fetch_add(t.n_full, 1);
+        t.full_of[o] = f;
+        t.row[f] = o;
       }
     }
   }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = fetch_add(t.ticket, 1) == (long long)gridDim.x - 1;
+    next_off = next_task = 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const long long full = __ldcg(t.n_full);
+  for (long long f0 = threadIdx.x & ~31u; f0 < full; f0 += blockDim.x) {
+    const long long f = f0 + lane, rest = f < full ? __ldcg(t.count + __ldcg(t.row + f)) - SLOTS : 0, pieces = (rest + PIECE - 1) / PIECE;
+    long long rest_sum = rest, piece_sum = pieces;     // up to and with this lane
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const long long a = __shfl_up_sync(0xffffffffu, rest_sum, d), b = __shfl_up_sync(0xffffffffu, piece_sum, d);
+      if (lane >= d) { rest_sum += a; piece_sum += b; }
+    }
+    long long off = 0, first = 0;
+    if (lane == 31) {
+      off = (long long)atomicAdd(&next_off, (unsigned long long)rest_sum);
+      first = (long long)atomicAdd(&next_task, (unsigned long long)piece_sum);
+    }
+    off = __shfl_sync(0xffffffffu, off, 31) + rest_sum - rest;
+    first = __shfl_sync(0xffffffffu, first, 31) + piece_sum - pieces;
+    if (f < full) { t.off[f] = off; t.done[f] = 0; }
+    for (long long i = 0; i < pieces; ++i) { t.task[2 * (first + i)] = f; t.task[2 * (first + i) + 1] = i; }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) *t.n_task = (long long)next_task;
+}
+
+template <bool VEC, typename T>
+__device__ __forceinline__ void load8(float* f, const T* s, int c, int cols) {
+  if (VEC) {
+    Vec8<T> v;
+    v.load(s + c);
+    v.to_float(f);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = c + j < cols ? to_f(s[c + j]) : 0.f;
+  }
+}
+template <bool VEC, typename T>
+__device__ __forceinline__ void store8(T* d, const float* f, int c, int cols) {
+  if (VEC) {
+    Vec8<T> v;
+    v.from_float(f);
+    v.store(d + c);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) if (c + j < cols) d[c + j] = from_f<T>(f[j]);
+  }
+}
+
+// The slots of every output row: the result, or, of a full row, the first value of its fp32 sum (acc [F, pitch]).  The first `fill` blocks
+// write the lists of the full rows.  weight (optional): one factor per source row
+template <typename T, bool VEC>
+__global__ void sum_slots_kernel(const T* __restrict__ src, const long long* __restrict__ idx, const float* __restrict__ weight, Tables tb,
+                                 T* __restrict__ out, float* __restrict__ acc, long long n, long long rows, int fill, int cols, int pitch) {
+  __shared__ long long slots[SLOTS];
+  if ((int)blockIdx.x < fill) {
+    if (*tb.n_full == 0) return;
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)fill * blockDim.x)
+      if (tb.pos[r] >= SLOTS) tb.list[tb.off[tb.full_of[idx[r]]] + tb.pos[r] - SLOTS] = r;
+    return;
+  }
+  for (long long o = (int)blockIdx.x - fill; o < rows; o += (int)gridDim.x - fill) {
+    const long long m = tb.count[o];
+    const int k = (int)(m < SLOTS ? m : SLOTS);
+    __syncthreads();                                   // slots is used again
+    if ((int)threadIdx.x < k) {                        // every slot ranked by its own thread
+      const long long mine = tb.slot[o * SLOTS + threadIdx.x];
+      int rank = 0;
+      for (int i = 0; i < k; ++i) rank += tb.slot[o * SLOTS + i] < mine ? 1 : 0;
+      slots[rank] = mine;
+    }
+    __syncthreads();
+    for (int c = (int)threadIdx.x * 8; c < cols; c += (int)blockDim.x * 8) {
+      float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int i = 0; i < k; ++i) {
+        const long long r = slots[i];
+        const float w = weight ? weight[r] : 1.f;
+        float f[8];
+        load8<VEC>(f, src + (size_t)r * cols, c, cols);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] = fmaf(f[j], w, sum[j]);
+      }
+      if (m <= SLOTS) {
+        store8<VEC>(out + (size_t)o * cols, sum, c, cols);
+      } else {
+        float4* d = reinterpret_cast<float4*>(acc + (size_t)tb.full_of[o] * pitch + c);
+        d[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+        d[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
+      }
+    }
+  }
+}
+
+// The pieces of the full rows, a block each.  An only piece meets the slots' sum here; several add to it by atomics, and the block that
+// adds the last one writes the result.
+template <typename T, bool VEC>
+__global__ void sum_pieces_kernel(const T* __restrict__ src, const float* __restrict__ weight, Tables tb, T* __restrict__ out, float* __restrict__ acc,
+                                  int cols, int pitch) {
+  __shared__ long long list[PIECE];
+  __shared__ bool last;
+  const long long tasks = *tb.n_task;
+  for (long long t = blockIdx.x; t < tasks; t += gridDim.x) {
+    const long long f = tb.task[2 * t], first = tb.task[2 * t + 1] * PIECE, o = tb.row[f], rest = tb.count[o] - SLOTS;
+    const int k = (int)min(rest - first, (long long)PIECE);
+    const bool alone = rest <= PIECE;
+    __syncthreads();                                   // list and last are used again
+    if ((int)threadIdx.x < k) list[threadIdx.x] = tb.list[tb.off[f] + first + threadIdx.x];
+    __syncthreads();
+    for (int c = (int)threadIdx.x * 8; c < cols; c += (int)blockDim.x * 8) {
+      float* d = acc + (size_t)f * pitch + c;
+      float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (alone) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] = d[j];
+      }
+#pragma unroll 4
+      for (int i = 0; i < k; ++i) {
+        const long long r = list[i];
+        const float w = weight ? weight[r] : 1.f;
+        float v[8];
+        load8<VEC>(v, src + (size_t)r * cols, c, cols);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] = fmaf(v[j], w, sum[j]);
+      }
+      if (alone) {
+        store8<VEC>(out + (size_t)o * cols, sum, c, cols);
+      } else {
+        atomicAdd(reinterpret_cast<float4*>(d), make_float4(sum[0], sum[1], sum[2], sum[3]));
+        atomicAdd(reinterpret_cast<float4*>(d + 4), make_float4(sum[4], sum[5], sum[6], sum[7]));
+      }
+    }
+    if (alone) continue;
+    __threadfence();                                   // this thread's share is in before the piece is counted
+    __syncthreads();
+    if (threadIdx.x == 0) last = fetch_add(tb.done + f, 1) == (rest + PIECE - 1) / PIECE - 1;
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      for (int c = (int)threadIdx.x * 8; c < cols; c += (int)blockDim.x * 8) {
+        const float4* d = reinterpret_cast<const float4*>(acc + (size_t)f * pitch + c);
+        const float4 a = __ldcg(d), b = __ldcg(d + 1);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        store8<VEC>(out + (size_t)o * cols, v, c, cols);
+      }
+    }
+  }
+}
+
+template <typename T, bool VEC>
+int launch_scatter_add(const T* src, const long long* idx, const float* weight, T* out, const Tables& tb, float* acc, long long n, long long rows,
+                       int cols, cudaStream_t s) {
+  const long long sms = msb::num_sms(), tasks = Tables::most_tasks(n, rows);
+  const int threads = cols >= 4096 ? 512 : cols >= 2048 ? 256 : 128, pitch = (cols + 7) / 8 * 8;
+  if (n > 0) {
+    place_rows_kernel<<<(int)min((n + 1023) / 1024, sms * 2), 1024, 0, s>>>(idx, tb, n);
+    MSB_CHECK_LAUNCH("place_rows");
+  }
+  const int fill = n > SLOTS ? (int)min((n + threads - 1) / threads, sms) : 0;
+  sum_slots_kernel<T, VEC><<<fill + (int)min(rows, sms * 32), threads, 0, s>>>(src, idx, weight, tb, out, acc, n, rows, fill, cols, pitch);
+  MSB_CHECK_LAUNCH("scatter_add_rows");
+  if (n > SLOTS) {
+    sum_pieces_kernel<T, VEC><<<(int)min(tasks, sms * (1536 / threads)), threads, 0, s>>>(src, weight, tb, out, acc, cols, pitch);
+    MSB_CHECK_LAUNCH("scatter_add_pieces");
+  }
+  return 0;
 }
 // out[idx[r]] += src[r] in fp32, for tables that are far larger than the rows that touch them (gradient of an embedding into its
 // accumulator): no dense gradient is formed, cleared, widened and added.  Rows may repeat often, so the sums are atomics, four
@@ -147,24 +285,21 @@ MSB_API int msb_gather_rows(const void* x, const long long* idx, void* out, long
   return 0;
 }
 // out [rows, cols] = for every source row r < n: out[idx[r]] += src[r] * (weight ? weight[r] : 1), summed in fp32; rows that no
-// source row names become zero.  chain: int64 scratch [10 rows + n].
-MSB_API int msb_scatter_add_rows(const void* src, const long long* idx, const float* weight, void* out, long long* chain, long long n, long long rows,
+// source row names become zero.  scratch, 16-byte aligned, with F = min(rows, n / 9): fp32 [F, cols rounded up to 8], then
+// int64 [10 rows + 3 + 5 F + 2 n + 2 (n / 32)].
+MSB_API int msb_scatter_add_rows(const void* src, const long long* idx, const float* weight, void* out, void* scratch, long long n, long long rows,
                                  int cols, int dtype, cudaStream_t s) {
   if (rows == 0 || cols == 0) return 0;
-  const Chains ch(chain, rows);
-  cudaError_t e = cudaMemsetAsync(ch.count, 0, (size_t)rows * sizeof(long long), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ch.head, 0xff, (size_t)rows * sizeof(long long), s);
+  float* acc = reinterpret_cast<float*>(scratch);
+  long long* tables = reinterpret_cast<long long*>(acc + Tables::most_full(n, rows) * ((cols + 7) / 8 * 8));
+  const Tables tb(tables, n, rows);
+  const cudaError_t e = cudaMemsetAsync(tables, 0, (size_t)(rows + 3) * sizeof(long long), s);
   if (e != cudaSuccess) { msb_set_error("scatter_add_rows: %s", cudaGetErrorString(e)); return 1; }
-  if (n > 0) {
-    const int cgrid = (int)(((n + 255) / 256) < (long long)msb::num_sms() * 8 ? (n + 255) / 256 : (long long)msb::num_sms() * 8);
-    chain_rows_kernel<<<cgrid, 256, 0, s>>>(idx, ch, n);
-    MSB_CHECK_LAUNCH("chain_rows");
-  }
-  const int vec = (cols % 8 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0) ? 1 : 0;
-  const int threads = cols >= 4096 ? 512 : cols >= 2048 ? 256 : 128;
-  const int grid = (int)(rows < (long long)msb::num_sms() * 32 ? rows : (long long)msb::num_sms() * 32);
-  MSB_DISPATCH_FLOAT(dtype, T, sum_chains_kernel<T><<<grid, threads, 0, s>>>((const T*)src, weight, ch, (T*)out, rows, cols, vec));
-  MSB_CHECK_LAUNCH("scatter_add_rows");
+  const bool vec = cols % 8 == 0 && (reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+  MSB_DISPATCH_FLOAT(dtype, T, {
+    return vec ? launch_scatter_add<T, true>((const T*)src, idx, weight, (T*)out, tb, acc, n, rows, cols, s)
+               : launch_scatter_add<T, false>((const T*)src, idx, weight, (T*)out, tb, acc, n, rows, cols, s);
+  });
   return 0;
 }
 // out [rows, cols] fp32: out[idx[r]] += src[r] for r < n with idx[r] >= 0.

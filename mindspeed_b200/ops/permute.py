@@ -32,10 +32,11 @@ class _Gather(torch.autograd.Function):
 def _scatter(src, idx, rows, weight):
     L = loader.require_lib()
     out = torch.empty(rows, src.shape[1], dtype=src.dtype, device=src.device)
-    chain = torch.empty(10 * rows + idx.numel(), dtype=torch.int64, device=src.device)
-    loader.check(L.msb_scatter_add_rows(loader.p(src), loader.p(idx), loader.p(weight), loader.p(out), loader.p(chain),
-                                        ctypes.c_longlong(idx.numel()), ctypes.c_longlong(rows), src.shape[1], code(src.dtype),
-                                        ctypes.c_void_p(loader.stream_ptr())), "scatter_add_rows")
+    n, cols = idx.numel(), src.shape[1]
+    full = min(rows, n // 9)                  # most output rows that more than eight source rows can name
+    scratch = torch.empty(full * ((cols + 7) // 8 * 4) + 10 * rows + 3 + 5 * full + 2 * n + 2 * (n // 32), dtype=torch.int64, device=src.device)
+    loader.check(L.msb_scatter_add_rows(loader.p(src), loader.p(idx), loader.p(weight), loader.p(out), loader.p(scratch), ctypes.c_longlong(n),
+                                        ctypes.c_longlong(rows), cols, code(src.dtype), ctypes.c_void_p(loader.stream_ptr())), "scatter_add_rows")
     return out
 
 

@@ -76,3 +76,45 @@ def test_add_rows_leaves_out_negative_rows():
     out = torch.zeros(3, 16, device="cuda")
     add_rows_(out, idx, src)
     assert out[:, 0].tolist() == [2.0, 0.0, 1.0] and not out.isnan().any()
+
+
+@pytest.mark.parametrize("n,rows,cols", [(9, 1, 8), (17, 2, 24), (4096, 1, 4096), (5000, 3, 133), (24576, 64, 264), (3000, 1000, 2048)])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_scatter_add_rows_with_many_repeats(n, rows, cols, weighted, dtype):
+    """More than eight source rows on an output row: eight in order, the others by atomics in any order.  fp32 sums of m terms in any order
+    are within m * 2^-23 of the sum of magnitudes, one rounding to the result's type follows."""
+    from mindspeed_b200.ops.permute import scatter_add_rows
+    torch.manual_seed(n + cols)
+    src = torch.randn(n, cols, device="cuda").to(dtype)
+    idx = torch.where(torch.rand(n, device="cuda") < 0.3, 0, torch.randint(0, rows, (n,), device="cuda"))
+    w = torch.rand(n, device="cuda") if weighted else None
+    terms = src.double() * (1.0 if w is None else w.double()[:, None])
+    zero = torch.zeros(rows, cols, device="cuda", dtype=torch.float64)
+    want, size = zero.index_add(0, idx, terms), zero.index_add(0, idx, terms.abs())
+    m = torch.bincount(idx, minlength=rows)[:, None]
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}[dtype]
+    for _ in range(2):                                # the second call meets used scratch
+        got = scatter_add_rows(src, idx, rows, w)
+        assert got.dtype == dtype
+        assert ((got.double() - want).abs() <= (m + 1) * 2.0 ** -23 * size + eps * want.abs() + 1e-7).all()
+
+
+def test_scatter_add_onto_one_row_is_not_serial():
+    """16384 rows on one output row and the same rows spread over 4096 (four each) move the same bytes.  The atomics of the former queue at
+    one row's addresses (at most five times the time); one thread that walks a list of them took a hundred times as long."""
+    from mindspeed_b200.ops.permute import scatter_add_rows
+    src = torch.randn(16384, 4096, device="cuda", dtype=torch.bfloat16)
+
+    def best(idx):
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            scatter_add_rows(src, idx, 4096)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times[1:])
+    spread = best(torch.arange(16384, device="cuda") % 4096)
+    assert best(torch.zeros(16384, dtype=torch.long, device="cuda")) < 20 * spread

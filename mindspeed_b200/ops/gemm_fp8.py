@@ -29,7 +29,8 @@ _ROW, _COL, _BLOCK = 1, 2, 4
 
 def _quant_ok(x, dtype):
     return (x.is_cuda and loader.lib() is not None and dtype in _FMT and x.dtype in (torch.bfloat16, torch.float16, torch.float32)
-            and x.is_contiguous() and x.data_ptr() % 16 == 0 and x.shape[1] % 128 == 0 and 0 < x.shape[0] < 2 ** 23)
+            and x.is_contiguous() and x.data_ptr() % 16 == 0 and x.shape[1] % 128 == 0 and x.shape[1] > 0
+            and 0 < x.shape[0] <= 65535 * 128)           # a grid's second dimension counts the 128-row tiles
 
 
 def _quant_kernel(x, form, dtype):

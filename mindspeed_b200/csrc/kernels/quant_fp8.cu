@@ -35,6 +35,13 @@ __device__ __forceinline__ float scale_of(uint32_t amax_bits, float inv_fmax) {
   const float a = __uint_as_float(amax_bits);
   return __fmul_rn(a < 1e-30f ? 1e-30f : a, inv_fmax);
 }
+// The quotient rounded to nearest, subnormal operands and results kept.  (The build flushes them to zero, in __fdiv_rn too.  PyTorch does
+// not, and under the smallest e5m2 scales, blocks below 1e-28, a subnormal value is not zero in fp8.)
+__device__ __forceinline__ float quotient(float v, float s) {
+  float q;
+  asm("div.rn.f32 %0, %1, %2;" : "=f"(q) : "f"(v), "f"(s));
+  return q;
+}
 template <bool E5M2>
 __device__ __forceinline__ uint2 to_fp8x8(const float* v) {
   uint32_t w[2];
@@ -116,7 +123,7 @@ __global__ void __launch_bounds__(256) quant_tile_kernel(QuantParams p) {
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[i][j] = __fdiv_rn(v[i][j], scale_blk);
+      for (int j = 0; j < 8; ++j) v[i][j] = quotient(v[i][j], scale_blk);
   }
   if (FORM & (Q_ROW | Q_BLOCK)) {
 #pragma unroll
@@ -129,7 +136,7 @@ __global__ void __launch_bounds__(256) quant_tile_kernel(QuantParams p) {
         const float s = scale_of(m, inv_fmax);
         if (cg == 0 && row0 + i < p.rows) p.s[(size_t)blockIdx.x * p.rows + row0 + i] = s;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = __fdiv_rn(v[i][j], s);
+        for (int j = 0; j < 8; ++j) o[j] = quotient(v[i][j], s);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = v[i][j];
@@ -143,7 +150,7 @@ __global__ void __launch_bounds__(256) quant_tile_kernel(QuantParams p) {
       float o[8];
       const float s = (FORM & Q_COL) ? col_scale[cg * 8 + j] : 1.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = (FORM & Q_COL) ? __fdiv_rn(v[i][j], s) : v[i][j];
+      for (int i = 0; i < 8; ++i) o[i] = (FORM & Q_COL) ? quotient(v[i][j], s) : v[i][j];
       // 8-byte unit rg of column 8 cg + j lies at unit rg ^ cg: the sixteen column groups of a store hit different banks
       *reinterpret_cast<uint2*>(tr + (cg * 8 + j) * QT + ((rg ^ cg) << 3)) = to_fp8x8<E5M2>(o);
     }

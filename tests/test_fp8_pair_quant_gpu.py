@@ -76,3 +76,28 @@ def test_pair_kernel_matches_reference(M, N, K, rowwise, out):
     G.check_status()
     tol = 4e-3 if out == "bf16" else 1e-3
     assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < tol
+
+
+@pytest.mark.parametrize("src", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("dtype", [torch.float8_e4m3fn, torch.float8_e5m2])
+def test_subnormal_values_are_not_flushed(src, dtype):
+    """Blocks whose largest value lies between 1e-42 and 1e-26: their subnormal values reach fp8 under the smallest scales (1e-30 / fmax
+    and a little above), bit for bit as in PyTorch, which keeps subnormals."""
+    from mindspeed_b200.ops import gemm_fp8 as F
+    from mindspeed_b200.ops.quant import quant_128x128, quant_1x128
+    torch.manual_seed(0)
+    size = torch.logspace(-42, -26, 256, device="cuda", dtype=torch.float64)
+    x = (torch.randn(256, 256, device="cuda", dtype=torch.float64) * size[:, None])
+    x[::2, ::3] = torch.randn(128, 86, device="cuda", dtype=torch.float64) * 5e-39
+    x = x.to(src)
+    tiny = (x != 0) & (x.abs().double() < 2.0 ** -126)
+    q, s, qt, st = F.quant_activation(x, dtype, rows=True, cols=True)
+    rq, rs = quant_1x128(x, dtype=dtype)
+    rqt, rst = quant_1x128(x.t().contiguous(), dtype=dtype)
+    for a, b in ((q, rq), (s, rs), (qt, rqt), (st, rst)):
+        _same(a, b)
+    if dtype == torch.float8_e5m2:
+        assert (q.float()[tiny] != 0).any()
+    else:
+        for a, b in zip(F.quant_weight(x), quant_128x128(x) + quant_128x128(x.t().contiguous())):
+            _same(a, b)

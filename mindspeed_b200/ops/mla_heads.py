@@ -32,10 +32,14 @@ def _rows_ok(t):
     return t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(st * e % 16 == 0 for st in t.stride()[:-1])
 
 
-def supports(q, kv, k_pe, cos, nope) -> bool:
+def supports(q, kv, k_pe, cos, sin, nope) -> bool:
     rope, vd = k_pe.shape[-1], kv.shape[-1] - nope
     return (loader.use_kernels(q) and q.dtype == kv.dtype == k_pe.dtype and q.dtype in CODE and q.numel() > 0
-            and nope % 8 == 0 and vd > 0 and vd % 8 == 0 and rope % 16 == 0 and 0 < rope <= 2048 and tuple(cos.shape) == (q.shape[0], rope))
+            and nope % 8 == 0 and vd > 0 and vd % 8 == 0 and rope % 16 == 0 and 0 < rope <= 2048
+            and kv.is_cuda and k_pe.is_cuda and cos.is_cuda and sin.is_cuda
+            # what the kernel indexes without asking: the same tokens and heads everywhere, one row of angles per position
+            and q.dim() == 4 and q.shape[3] == nope + rope and kv.shape[:3] == q.shape[:3] and k_pe.shape[:-1] == q.shape[:2]
+            and tuple(cos.shape) == tuple(sin.shape) == (q.shape[0], rope))
 
 
 class _MlaHeads(torch.autograd.Function):
@@ -71,6 +75,6 @@ class _MlaHeads(torch.autograd.Function):
 
 
 def mla_heads(q, kv, k_pe, cos, sin, nope, interleaved=False):
-    if supports(q, kv, k_pe, cos, nope):
+    if supports(q, kv, k_pe, cos, sin, nope):
         return _MlaHeads.apply(q, kv, k_pe, cos.float().contiguous(), sin.float().contiguous(), nope, bool(interleaved))
     return mla_heads_ref(q, kv, k_pe, cos, sin, nope, interleaved)

@@ -11,6 +11,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include "msb_launch.hpp"
+
 #define MSB_API extern "C" __attribute__((visibility("default")))
 
 // dtype codes shared with python (mindspeed_b200/ops/_dtypes.py)

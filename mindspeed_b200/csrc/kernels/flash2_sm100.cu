@@ -381,12 +381,8 @@ MSB_API int msb_flash_fwd2(const void* q, const void* k, const void* v, void* o,
   p.O = (__nv_bfloat16*)o; p.lse = lse;
   p.sq = sq; p.sk = sk; p.b = b; p.nq = nq; p.nkv = nkv; p.causal = causal; p.q_offset = q_offset;
   p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(flash_fwd2_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd2Smem::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("flash_fwd2: cannot set dynamic shared memory: %s", cudaGetErrorString(e)); return 1; }
-    attr = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)flash_fwd2_sm100_kernel, Fwd2Smem::TOTAL, "flash_fwd2", stated)) return bad;
   // A group is as many heads as have their K and V in half of L2 (48 MB): every CTA that runs at a time then streams from L2, and the
   // group is wide enough that its shortest CTAs end the launch.  s = 4096, 32 / 8 heads, one head after the other: an SM was busy for
   // three quarters of the launch.
@@ -956,12 +952,8 @@ MSB_API int msb_flash_bwd(const void* q, const void* k, const void* v, const voi
   p.nlse2 = nlse2; p.ndelta = ndelta;
   p.sq = sq; p.sk = sk; p.b = b; p.nq = nq; p.nkv = nkv; p.sq_pad = sq_pad; p.causal = causal; p.q_offset = q_offset;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(flash_bwd_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmem::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("flash_bwd: cannot set dynamic shared memory: %s", cudaGetErrorString(e)); return 1; }
-    attr = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)flash_bwd_sm100_kernel, BwdSmem::TOTAL, "flash_bwd", stated)) return bad;
   const long long ctas = (long long)(split_heads ? nq : nkv) * ((sk + FB - 1) / FB);
   MSB_REQUIRE(ctas <= 0x7fffffffll, "flash_bwd: grid too large (%lld)", ctas);
   dim3 grid((unsigned)ctas, 1, b);

@@ -256,12 +256,8 @@ MSB_API int msb_flash_fwd(const void* q, const void* k, const void* v, void* o, 
   p.O = (__nv_bfloat16*)o; p.lse = lse;
   p.sq = sq; p.sk = sk; p.b = b; p.nq = nq; p.nkv = nkv; p.causal = causal; p.q_offset = q_offset;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(flash_fwd_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashSmem::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("flash_fwd: cannot set dynamic shared memory: %s", cudaGetErrorString(e)); return 1; }
-    attr = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)flash_fwd_sm100_kernel, FlashSmem::TOTAL, "flash_fwd", stated)) return bad;
   dim3 grid((sq + FB - 1) / FB, nq, b);
   flash_fwd_sm100_kernel<<<grid, 192, FlashSmem::TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("flash_fwd_sm100");

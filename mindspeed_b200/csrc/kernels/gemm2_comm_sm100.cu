@@ -511,12 +511,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(224, 1) gemm2_comm_k
 template <int MODE, bool B_MN>
 int launch_comm2(const Comm2Params& p, int pairs, cudaStream_t s) {
   auto kern = gemm2_comm_kernel<MODE, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("gemm2_comm: cannot set %d bytes of dynamic shared memory: %s", Smem::TOTAL, cudaGetErrorString(e)); return 1; }
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)kern, Smem::TOTAL, "gemm2_comm", stated)) return bad;
   kern<<<2 * pairs, 224, Smem::TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("gemm2_comm");
   return 0;

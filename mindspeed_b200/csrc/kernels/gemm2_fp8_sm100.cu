@@ -278,12 +278,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1) gemm2_
 template <int EPI, bool B_ROWWISE>
 int launch_pair(const Fp8PairParams& p, int pairs, cudaStream_t s) {
   auto kern = gemm2_fp8_kernel<EPI, B_ROWWISE>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
-    if (e != cudaSuccess) { msb_set_error("gemm2_fp8: cannot set %d bytes of dynamic shared memory: %s", P_SMEM, cudaGetErrorString(e)); return 1; }
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)kern, P_SMEM, "gemm2_fp8", stated)) return bad;
   kern<<<2 * pairs, P_THREADS, P_SMEM, s>>>(p);
   MSB_CHECK_LAUNCH("gemm2_fp8");
   return 0;

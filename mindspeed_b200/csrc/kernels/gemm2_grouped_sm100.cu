@@ -354,12 +354,8 @@ template <int NSTAGE, int MODE, int EPI, bool B_MN>
 int launch_grouped(const GroupedParams& p, int pairs, cudaStream_t s) {
   using L = SmemG<NSTAGE, EPI>;
   auto kern = gemm2_grouped_kernel<NSTAGE, MODE, EPI, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("gemm2_grouped: cannot set %d bytes of dynamic shared memory: %s", L::TOTAL, cudaGetErrorString(e)); return 1; }
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)kern, L::TOTAL, "gemm2_grouped", stated)) return bad;
   kern<<<2 * pairs, 192, L::TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("gemm2_grouped");
   return 0;

@@ -308,12 +308,8 @@ template <int BN, int NSTAGE, int EPI, bool A_MN, bool B_MN>
 int launch2_variant(const Gemm2Params& p, int pairs, cudaStream_t s) {
   using L = Smem2<BN, NSTAGE, EPI>;
   auto kern = gemm2_sm100_kernel<BN, NSTAGE, EPI, A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("gemm2_sm100: cannot set %d bytes of dynamic shared memory: %s", L::TOTAL, cudaGetErrorString(e)); return 1; }
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)kern, L::TOTAL, "gemm2_sm100", stated)) return bad;
   kern<<<2 * pairs, 192, L::TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("gemm2_sm100");
   return 0;

@@ -292,12 +292,8 @@ bool pair_kernel_fits(const void* D, const float* sB, int M, int N, int b_scale_
 template <int EPI>
 int launch_fp8(const Fp8Params& p, int grid, cudaStream_t s) {
   auto kern = gemm_fp8_blockscaled_kernel<EPI>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
-    if (e != cudaSuccess) { msb_set_error("gemm_fp8: cannot set %d bytes of dynamic shared memory: %s", SMEM_TOTAL, cudaGetErrorString(e)); return 1; }
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)kern, SMEM_TOTAL, "gemm_fp8", stated)) return bad;
   kern<<<grid, 320, SMEM_TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("gemm_fp8_blockscaled");
   return 0;

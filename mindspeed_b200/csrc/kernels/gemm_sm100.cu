@@ -677,12 +677,8 @@ template <int BN, int NSTAGE, int MODE, bool B_MN>
 int launch_comm_variant(const CommParams& cp, int grid, cudaStream_t s) {
   using L = SmemLayout<BN, NSTAGE>;
   auto kern = gemm_comm_sm100_kernel<BN, NSTAGE, MODE, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("gemm_comm_sm100: cannot set %d bytes of dynamic shared memory: %s", L::TOTAL, cudaGetErrorString(e)); return 1; }
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)kern, L::TOTAL, "gemm_comm_sm100", stated)) return bad;
   kern<<<grid, 448, L::TOTAL, s>>>(cp);
   MSB_CHECK_LAUNCH("gemm_comm_sm100");
   return 0;
@@ -692,12 +688,8 @@ template <int BN, int NSTAGE, int EPI, bool A_MN, bool B_MN>
 int launch_variant(const GemmParams& p, int grid, cudaStream_t s) {
   using L = SmemLayout<BN, NSTAGE>;
   auto kern = gemm_sm100_kernel<BN, NSTAGE, EPI, A_MN, B_MN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) { msb_set_error("gemm_sm100: cannot set %d bytes of dynamic shared memory: %s", L::TOTAL, cudaGetErrorString(e)); return 1; }
-    attr_set = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)kern, L::TOTAL, "gemm_sm100", stated)) return bad;
   kern<<<grid, 192, L::TOTAL, s>>>(p);
   MSB_CHECK_LAUNCH("gemm_sm100");
   return 0;

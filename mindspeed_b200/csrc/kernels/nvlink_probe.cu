@@ -115,11 +115,8 @@ MSB_API int msb_nvlink_probe(const void* src, void* const* peer, size_t bytes, i
   for (int i = 0; i < 8; ++i) p.peer[i] = i < world ? (uint8_t*)peer[i] : nullptr;
   p.bytes = bytes; p.chunk = chunk; p.world = world; p.rank = rank; p.spread = spread; p.mode = mode; p.ring = ring; p.status = status;
   const int smem = 8 * 16384 + 64 + 1024;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(nvlink_probe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attr = true;
-  }
+  static std::atomic<unsigned long long> stated{0};
+  if (int bad = msb::allow_smem((const void*)nvlink_probe_kernel, smem, "nvlink_probe", stated)) return bad;
   nvlink_probe_kernel<<<ctas > 0 ? ctas : msb::num_sms(), 256, smem, s>>>(p);
   MSB_CHECK_LAUNCH("nvlink_probe");
   return 0;

@@ -78,6 +78,49 @@ def test_pair_kernel_matches_reference(M, N, K, rowwise, out):
     assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < tol
 
 
+@pytest.mark.parametrize("M,N,K", [(300, 201, 640), (1, 130, 128), (129, 1, 1152), (2304, 2049, 256)])
+@pytest.mark.parametrize("out", ["bf16", "f32", "acc"])
+def test_rows_that_tma_cannot_store_take_the_single_cta_kernel(M, N, K, out):
+    """Row-wise scales and N % 4 != 0: neither the output's rows nor the scales start on 16-byte boundaries.  Bounds as above."""
+    from mindspeed_b200.ops import gemm as G
+    from mindspeed_b200.ops import gemm_fp8 as F
+    from mindspeed_b200.ops.quant import quant_1x128
+    torch.manual_seed(M + N)
+    xq, xs = quant_1x128(torch.randn(M, K, device="cuda") * torch.rand(M, 1, device="cuda"), dtype=torch.float8_e5m2)
+    wq, ws = quant_1x128(torch.randn(N, K, device="cuda") * torch.rand(N, 1, device="cuda"))
+    ref = F._ref(xq, xs, wq, ws, True, torch.float32)
+    guard = torch.full((M * N + 64,), 7.0, device="cuda", dtype=torch.bfloat16 if out == "bf16" else torch.float32)
+    y = guard[:M * N].view(M, N)
+    if out == "acc":
+        y.copy_(torch.randn(M, N, device="cuda"))
+        ref = ref + y
+    F.fp8_gemm(xq, xs, wq, ws, w_rowwise=True, out=y, accumulate=out == "acc")
+    torch.cuda.synchronize()
+    G.check_status()
+    tol = 4e-3 if out == "bf16" else 1e-3
+    assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < tol
+    assert (guard[M * N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("rowwise", [False, True])
+def test_output_columns_of_a_wider_matrix(rowwise):
+    """Rows of an fp32 output that start 4 bytes past a 16-byte boundary, in a matrix large enough for the pair kernel."""
+    from mindspeed_b200.ops import gemm as G
+    from mindspeed_b200.ops import gemm_fp8 as F
+    from mindspeed_b200.ops.quant import quant_128x128, quant_1x128
+    torch.manual_seed(5)
+    xq, xs = quant_1x128(torch.randn(2048, 256, device="cuda"))
+    w = torch.randn(2304, 256, device="cuda")
+    wq, ws = quant_1x128(w) if rowwise else quant_128x128(w)
+    wide = torch.full((2048, 2304 + 5), 7.0, device="cuda")
+    F.fp8_gemm(xq, xs, wq, ws, w_rowwise=rowwise, out=wide[:, 1:2305])
+    torch.cuda.synchronize()
+    G.check_status()
+    ref = F._ref(xq, xs, wq, ws, rowwise, torch.float32)
+    assert ((wide[:, 1:2305] - ref).abs().max() / ref.abs().max()).item() < 1e-3
+    assert (wide[:, 0] == 7.0).all() and (wide[:, 2305:] == 7.0).all()
+
+
 @pytest.mark.parametrize("src", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("dtype", [torch.float8_e4m3fn, torch.float8_e5m2])
 def test_subnormal_values_are_not_flushed(src, dtype):

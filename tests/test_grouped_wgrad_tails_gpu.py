@@ -26,3 +26,30 @@ def test_wgrad_adds_every_row_once(counts, K, N):
     torch.cuda.synchronize()
     G.check_status()
     assert ((acc - want).abs().max() / want.abs().max()).item() < 1e-5
+
+
+@pytest.mark.parametrize("epilogue", [0, 1])
+def test_wgrad_stores(epilogue):
+    """The storing forms (bf16, fp32): every expert with rows is written, the others keep what they hold."""
+    import ctypes
+
+    from mindspeed_b200.ops import gemm as G
+    from mindspeed_b200.ops import loader
+    from mindspeed_b200.ops.grouped_gemm import TAIL, _offsets
+    torch.manual_seed(epilogue)
+    counts, K, N = [70, 0, 1, 64], 264, 136
+    rows = sum(counts)
+    x, dy = (torch.randn(rows, c, device="cuda").bfloat16() for c in (K, N))
+    offs = _offsets(counts, x.device)
+    dw = torch.full((len(counts), K, N), 7.0, device="cuda", dtype=(torch.bfloat16, torch.float32)[epilogue])
+    xt, dyt = (torch.empty(len(counts) * TAIL, c, device="cuda", dtype=torch.bfloat16) for c in (K, N))
+    loader.check(loader.require_lib().msb_grouped_gemm_wgrad(
+        loader.p(x), loader.p(dy), loader.p(dw), loader.p(offs), loader.p(xt), loader.p(dyt), len(counts), rows, K, N, epilogue,
+        loader.p(G.status_word(x.device)), ctypes.c_void_p(loader.stream_ptr())), "grouped_gemm_wgrad")
+    torch.cuda.synchronize()
+    G.check_status()
+    s = 0
+    for e, n in enumerate(counts):
+        want = (x[s:s + n].double().t() @ dy[s:s + n].double()) if n else torch.full((K, N), 7.0, device="cuda", dtype=torch.float64)
+        s += n
+        assert ((dw[e].double() - want).abs().max() / want.abs().max()).item() < (2.0 ** -8 if epilogue == 0 else 1e-5)

@@ -5,6 +5,10 @@
   python -m mindspeed_b200.benchmarks.ncu_targets fp8         # 3 launches of the block-scaled fp8 GEMM, 8192 x 8192 x 8192
   python -m mindspeed_b200.benchmarks.ncu_targets gemm_tp8    # the four forward GEMM shapes of a Llama-3-8B layer at TP8
   python -m mindspeed_b200.benchmarks.ncu_targets flash       # 2 launches each of flash-attention forward and backward
+  python -m mindspeed_b200.benchmarks.ncu_targets quant       # fp8 quantiser, 4096 x 28672 bf16: row, both and block forms
+  python -m mindspeed_b200.benchmarks.ncu_targets fp8_wgrad   # 2 launches of the fp8 GEMM with row-wise scales on both sides
+  python -m mindspeed_b200.benchmarks.ncu_targets grouped     # grouped expert GEMMs, 64 experts of about 384 rows: fwd / dgrad / wgrad
+  python -m mindspeed_b200.benchmarks.ncu_targets mla_heads   # latent-attention head kernels, forward and backward
 
 Inputs exceed the 126 MB L2 but stay well under 2 GB on the device; there are only a handful of launches, so a
 ``--set full`` capture ends by itself within a minute or two.
@@ -93,10 +97,10 @@ def gemm_tp8():
 
 
 def flash():
-    """Two launches each of the flash-attention forward and backward kernels: seq 4096, 8 query / 2 KV heads, causal."""
+    """Two launches each of the flash-attention forward and backward kernels: seq 4096, 32 query / 8 KV heads, causal."""
     from ..ops import gemm as G
     from ..ops.flash_sm100_impl import flash_bwd, flash_fwd
-    s, nq, nkv = 4096, 8, 2
+    s, nq, nkv = 4096, 32, 8
     q = torch.randn(s, 1, nq, 128, device="cuda", dtype=torch.bfloat16)
     k = torch.randn(s, 1, nkv, 128, device="cuda", dtype=torch.bfloat16)
     v = torch.randn(s, 1, nkv, 128, device="cuda", dtype=torch.bfloat16)
@@ -108,5 +112,55 @@ def flash():
     G.check_status()
 
 
+def quant():
+    from ..ops import gemm_fp8 as F
+    x = torch.randn(4096, 28672, device="cuda", dtype=torch.bfloat16)
+    for _ in range(2):
+        F.quant_activation(x)
+        F.quant_activation(x, cols=True)
+        F.quant_weight(x)
+    torch.cuda.synchronize()
+
+
+def fp8_wgrad():
+    """dW of a 4096 -> 28672 layer from 4096 tokens."""
+    from ..ops import gemm as G
+    from ..ops import gemm_fp8 as F
+    _, _, dyq, dys = F.quant_activation(torch.randn(4096, 28672, device="cuda", dtype=torch.bfloat16), rows=False, cols=True)
+    _, _, xq, xs = F.quant_activation(torch.randn(4096, 4096, device="cuda", dtype=torch.bfloat16), rows=False, cols=True)
+    for _ in range(2):
+        F.fp8_gemm(dyq, dys, xq, xs, w_rowwise=True)
+    torch.cuda.synchronize()
+    G.check_status()
+
+
+def grouped():
+    from ..ops import gemm as G
+    from ..ops.grouped_gemm import grouped_gemm
+    E, rows, K, N = 64, 24576, 2048, 3072
+    x = torch.randn(rows, K, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    w = torch.randn(E, K, N, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    w.main_grad = torch.zeros(E, K, N, device="cuda")
+    counts = torch.full((E,), rows // E, device="cuda", dtype=torch.int64)
+    counts[::2] += 23
+    counts[1::2] -= 23
+    for _ in range(2):
+        grouped_gemm(x, w, counts).backward(torch.ones(rows, N, device="cuda", dtype=torch.bfloat16))
+    torch.cuda.synchronize()
+    G.check_status()
+
+
+def mla_heads():
+    from ..ops.mla_heads import mla_heads as heads
+    s, n, nope, rope, vd = 4096, 32, 128, 64, 128
+    q, kv, pe = (torch.randn(s, 1, *shape, device="cuda", dtype=torch.bfloat16, requires_grad=True) for shape in ((n, nope + rope), (n, nope + vd), (rope,)))
+    ang = torch.randn(s, rope, device="cuda")
+    for _ in range(2):
+        out = heads(q, kv, pe, ang.cos(), ang.sin(), nope)
+        torch.autograd.backward(out, [torch.ones_like(t) for t in out])
+    torch.cuda.synchronize()
+
+
 if __name__ == "__main__":
-    {"gemm": gemm, "elementwise": elementwise, "fp8": fp8, "gemm_tp8": gemm_tp8, "flash": flash}[sys.argv[1] if len(sys.argv) > 1 else "gemm"]()
+    {"gemm": gemm, "elementwise": elementwise, "fp8": fp8, "gemm_tp8": gemm_tp8, "flash": flash, "quant": quant, "fp8_wgrad": fp8_wgrad,
+     "grouped": grouped, "mla_heads": mla_heads}[sys.argv[1] if len(sys.argv) > 1 else "gemm"]()

@@ -9,12 +9,13 @@
 //                       S0 S1 | PV0 S0' | PV1 S1' | ...   so tile t's softmax overlaps the other tile's MMAs
 //   warps 0-3 / 4-7     softmax of tile 0 / tile 1, one thread per query row: row maximum (four chains of three-input maxima), exp2,
 //                       row sum, P -> TMEM.  They hold a whole score row per thread (setmaxnreg).
-//   The issuing thread is what bounds it, a softmax warp waits a third of the time: a barrier costs it 75 to 150 cycles, done or
-//   not.  One commit frees K and V, the scores' commit stands for P V as well, descriptors are one addition each.  s = 8192, 32 / 8
-//   heads, causal: 573 us at first, 521 with the softmax above, 487 with the heaviest tiles first, 468 with this issue.
 //                       O stays in tensor memory; it is rescaled only when the running maximum grew by more than 2^8
 //                       since the last rescale (the stale maximum is used for P meanwhile, which stays within range),
 //                       so most key tiles never touch O.
+// The issuing thread is what bounds it, a softmax warp waits a third of the time: a barrier costs it 75 to 150 cycles, done or
+// not.  One commit frees K and V, the scores' commit stands for P V as well, descriptors are one addition each.  s = 8192, 32 / 8
+// heads, causal: 573 us at first, 521 with the softmax above, 487 with the heaviest tiles first, 468 with this issue (474 with the row
+// sum in the order of the keys).
 // Epilogue: O / l -> bf16 -> shared memory (the tile's Q buffer) -> TMA store; LSE (natural log) to global memory.
 // reference semantics: torch_npu.npu_fusion_attention returning softmax max/sum
 // (mindspeed/core/transformer/flash_attention/flash_attention/adaptor.py:21-85, mindspeed/ops/fusion_attention_v2.py:22-114).
@@ -132,87 +133,87 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
 
   // registers of the launch: 384 x 168 = 64512; the two softmax warpgroups hold a whole score row per thread
   if (warp >= 8) {       // warps 10 and 11 only complete the warpgroup that gives registers away
-   asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-   if (warp == 8) {
-    // ===================== TMA producer =====================
-    if (lane == 0 && n_max > 0) {
-      mbar_arrive_expect_tx(q_full, 2 * TILE_BYTES);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const uint32_t qs = base + Fwd2Smem::Q_OFF + t * TILE_BYTES;
-        tma_load_5d(qs, &p.tmQ, q_full, 0, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
-        tma_load_5d(qs + HALF_BYTES, &p.tmQ, q_full, 64, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
-      }
-      auto load = [&](uint32_t dst, const CUtensorMap* tm, uint32_t full, int j) {
-        mbar_arrive_expect_tx(full, TILE_BYTES);
-        tma_load_4d(dst, tm, full, 0, kv_head, batch, j * FB);
-        tma_load_4d(dst + HALF_BYTES, tm, full, 64, kv_head, batch, j * FB);
-      };
-      auto load_k = [&](int j) { if (j < n_max) load(base + Fwd2Smem::K_OFF + (j & 1) * TILE_BYTES, &p.tmK, k_full(j & 1), j); };
-      auto load_v = [&](int j) { if (j < n_max) load(base + Fwd2Smem::V_OFF + (j & 1) * TILE_BYTES, &p.tmV, v_full(j & 1), j); };
-      load_k(0); load_v(0); load_k(1); load_v(1);
-      // kv_free(c & 1): the scores of key tile c and P V of tile c - 1 are done, so K_c and V_c-1 may be overwritten.  Two barriers in
-      // turn: the one after next needs tiles that are only loaded here, so no phase can pass unseen.
-      for (int c = 0; c + 1 < n_max; ++c) {
-        if (!mbar_wait(kv_free(c & 1), (uint32_t)((c >> 1) & 1), p.status, 0x310u)) break;
-        if (c > 0) load_v(c + 1);
-        load_k(c + 2);
-      }
-    }
-   } else if (warp == 9) {
-    // ===================== MMA issuer =====================
-    if (lane == 0 && n_max > 0) {
-      constexpr uint32_t idesc_qk = make_idesc_f16(128, 128, 1, 0, 0);
-      constexpr uint32_t idesc_pv = make_idesc_f16(128, 128, 1, 0, 1);
-      // descriptors of tile 0 / stage 0; an address grows by 16-byte units in the low word
-      const uint64_t qd = make_smem_desc(base + Fwd2Smem::Q_OFF, 0, 1024), kd = make_smem_desc(base + Fwd2Smem::K_OFF, 0, 1024);
-      const uint64_t vd = make_smem_desc(base + Fwd2Smem::V_OFF, HALF_BYTES, 1024);
-      auto wait = [&](uint32_t b, uint32_t parity, unsigned int code) {
-        const bool ok = mbar_wait(b, parity, p.status, code);
-        tc_fence_after();
-        return ok;
-      };
-      auto issue_s = [&](int t, int j) {
-        const uint64_t q0d = qd + (uint64_t)(t * (TILE_BYTES >> 4)), k0d = kd + (uint64_t)((j & 1) * (TILE_BYTES >> 4));
-#pragma unroll
-        for (int k = 0; k < FD / 16; ++k) {
-          const uint64_t off = (uint64_t)(((k >> 2) * HALF_BYTES + (k & 3) * 32) >> 4);
-          umma_f16(tmem_base + (uint32_t)(t * 128), q0d + off, k0d + off, idesc_qk, k ? 1u : 0u);
-        }
-        umma_commit(s_full(t));       // completes after everything issued before: P V of the last key tile is in O as well
-      };
-      auto issue_pv = [&](int t, int j) {
-        const uint64_t v0d = vd + (uint64_t)((j & 1) * (TILE_BYTES >> 4));
-        const uint32_t tP = tmem_base + (uint32_t)(t * 128), tO = tmem_base + 256u + (uint32_t)(t * 128);
-#pragma unroll
-        for (int k = 0; k < FB / 16; ++k)      // MN-major: 16 keys = 2048 B; 16 bf16 of P = 8 columns
-          umma_f16_ts(tO, tP + (uint32_t)(k * 8), v0d + (uint64_t)(k * (16 * 128 >> 4)), idesc_pv, (j | k) ? 1u : 0u);
-      };
-      bool ok = wait(q_full, 0, 0x320u);
-      if (ok) ok = wait(k_full(0), 0, 0x321u);
-      if (ok) {
-        if (n_t[0] > 0) issue_s(0, 0);
-        if (n_t[1] > 0) issue_s(1, 0);
-        umma_commit(kv_free(0));
-      }
-      for (int j = 0; j < n_max && ok; ++j) {
-        const uint32_t ph = (uint32_t)((j >> 1) & 1), jp = (uint32_t)(j & 1);
-        if (!(ok = wait(v_full(j & 1), ph, 0x322u))) break;
-        if (j + 1 < n_max && !(ok = wait(k_full((j + 1) & 1), (uint32_t)(((j + 1) >> 1) & 1), 0x324u))) break;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    if (warp == 8) {
+      // ===================== TMA producer =====================
+      if (lane == 0 && n_max > 0) {
+        mbar_arrive_expect_tx(q_full, 2 * TILE_BYTES);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          if (j < n_t[t]) {
-            if (!(ok = wait(p_full(t), jp, 0x323u))) break;
-            issue_pv(t, j);
-          }
-          if (j + 1 < n_t[t]) issue_s(t, j + 1);
+          const uint32_t qs = base + Fwd2Smem::Q_OFF + t * TILE_BYTES;
+          tma_load_5d(qs, &p.tmQ, q_full, 0, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
+          tma_load_5d(qs + HALF_BYTES, &p.tmQ, q_full, 64, head - kv_head * (p.nq / p.nkv), kv_head, batch, q0 + t * FB);
         }
-        if (!ok) break;
-        umma_commit(kv_free((j + 1) & 1));
+        auto load = [&](uint32_t dst, const CUtensorMap* tm, uint32_t full, int j) {
+          mbar_arrive_expect_tx(full, TILE_BYTES);
+          tma_load_4d(dst, tm, full, 0, kv_head, batch, j * FB);
+          tma_load_4d(dst + HALF_BYTES, tm, full, 64, kv_head, batch, j * FB);
+        };
+        auto load_k = [&](int j) { if (j < n_max) load(base + Fwd2Smem::K_OFF + (j & 1) * TILE_BYTES, &p.tmK, k_full(j & 1), j); };
+        auto load_v = [&](int j) { if (j < n_max) load(base + Fwd2Smem::V_OFF + (j & 1) * TILE_BYTES, &p.tmV, v_full(j & 1), j); };
+        load_k(0); load_v(0); load_k(1); load_v(1);
+        // kv_free(c & 1): the scores of key tile c and P V of tile c - 1 are done, so K_c and V_c-1 may be overwritten.  Two barriers in
+        // turn: the one after next needs tiles that are only loaded here, so no phase can pass unseen.
+        for (int c = 0; c + 1 < n_max; ++c) {
+          if (!mbar_wait(kv_free(c & 1), (uint32_t)((c >> 1) & 1), p.status, 0x310u)) break;
+          if (c > 0) load_v(c + 1);
+          load_k(c + 2);
+        }
       }
-      if (ok) umma_commit(o_done);
+    } else if (warp == 9) {
+      // ===================== MMA issuer =====================
+      if (lane == 0 && n_max > 0) {
+        constexpr uint32_t idesc_qk = make_idesc_f16(128, 128, 1, 0, 0);
+        constexpr uint32_t idesc_pv = make_idesc_f16(128, 128, 1, 0, 1);
+        // descriptors of tile 0 / stage 0; an address grows by 16-byte units in the low word
+        const uint64_t qd = make_smem_desc(base + Fwd2Smem::Q_OFF, 0, 1024), kd = make_smem_desc(base + Fwd2Smem::K_OFF, 0, 1024);
+        const uint64_t vd = make_smem_desc(base + Fwd2Smem::V_OFF, HALF_BYTES, 1024);
+        auto wait = [&](uint32_t b, uint32_t parity, unsigned int code) {
+          const bool ok = mbar_wait(b, parity, p.status, code);
+          tc_fence_after();
+          return ok;
+        };
+        auto issue_s = [&](int t, int j) {
+          const uint64_t q0d = qd + (uint64_t)(t * (TILE_BYTES >> 4)), k0d = kd + (uint64_t)((j & 1) * (TILE_BYTES >> 4));
+#pragma unroll
+          for (int k = 0; k < FD / 16; ++k) {
+            const uint64_t off = (uint64_t)(((k >> 2) * HALF_BYTES + (k & 3) * 32) >> 4);
+            umma_f16(tmem_base + (uint32_t)(t * 128), q0d + off, k0d + off, idesc_qk, k ? 1u : 0u);
+          }
+          umma_commit(s_full(t));       // completes after everything issued before: P V of the last key tile is in O as well
+        };
+        auto issue_pv = [&](int t, int j) {
+          const uint64_t v0d = vd + (uint64_t)((j & 1) * (TILE_BYTES >> 4));
+          const uint32_t tP = tmem_base + (uint32_t)(t * 128), tO = tmem_base + 256u + (uint32_t)(t * 128);
+#pragma unroll
+          for (int k = 0; k < FB / 16; ++k)      // MN-major: 16 keys = 2048 B; 16 bf16 of P = 8 columns
+            umma_f16_ts(tO, tP + (uint32_t)(k * 8), v0d + (uint64_t)(k * (16 * 128 >> 4)), idesc_pv, (j | k) ? 1u : 0u);
+        };
+        bool ok = wait(q_full, 0, 0x320u);
+        if (ok) ok = wait(k_full(0), 0, 0x321u);
+        if (ok) {
+          if (n_t[0] > 0) issue_s(0, 0);
+          if (n_t[1] > 0) issue_s(1, 0);
+          umma_commit(kv_free(0));
+        }
+        for (int j = 0; j < n_max && ok; ++j) {
+          const uint32_t ph = (uint32_t)((j >> 1) & 1), jp = (uint32_t)(j & 1);
+          if (!(ok = wait(v_full(j & 1), ph, 0x322u))) break;
+          if (j + 1 < n_max && !(ok = wait(k_full((j + 1) & 1), (uint32_t)(((j + 1) >> 1) & 1), 0x324u))) break;
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (j < n_t[t]) {
+              if (!(ok = wait(p_full(t), jp, 0x323u))) break;
+              issue_pv(t, j);
+            }
+            if (j + 1 < n_t[t]) issue_s(t, j + 1);
+          }
+          if (!ok) break;
+          umma_commit(kv_free((j + 1) & 1));
+        }
+        if (ok) umma_commit(o_done);
+      }
     }
-   }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");     // 256 x 208 + 128 x 80 = 63488
     // ===================== softmax (warps 0-3: tile 0, warps 4-7: tile 1) =====================
@@ -275,8 +276,9 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) flash_fwd2_sm100_kernel(const 
       const float m_ref = (m_used == -INFINITY) ? 0.f : m_used;
       // probabilities -> packed bf16 over the first 64 columns of S, row sum (masked scores are -inf -> 0)
       const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), nref2 = pack_f32x2(-m_ref, -m_ref);
-      // the row sum keeps the order of the keys, pair after pair, as the log-sum-exp's last bits always had it; its chain of 64 additions
-      // is shorter than the exponentials of the row
+      // The row sum takes the keys in order, pair after pair: the log-sum-exp's last bits, and with them bf16 roundings of the output, show
+      // the order.  (Four interleaved chains of packed additions: 463 us instead of 474 at s = 8192, 32 / 8 heads, causal.  Summed
+      // after P is handed over: no difference.)
       float l_tile = 0.f;
 #pragma unroll
       for (int c = 0; c < FB; c += 32) {
@@ -420,8 +422,8 @@ MSB_API int msb_flash_fwd2(const void* q, const void* k, const void* v, void* o,
 //                 P^T = exp2(S^T scale log2e - LSE log2e), dS^T = P^T (dP^T - delta), two lanes of arithmetic per instruction, the
 //                 statistics of a column by broadcast reads of shared memory
 //   warps 10-13   dQ: tensor memory -> softmax scale -> staging -> TMA reduce-add into the fp32 dQ
-// Bound: shared memory moves 490 KB per 128 x 128 tile (operands 290, TMA writes 64, dS 32, dQ staging in and out 128), 3840 cycles at
-// 128 B a cycle, beside 2560 cycles of MMA.  Measured at s = 8192, 32 / 8 heads, causal: 2173 us with one tile in flight and four
+// Bound: shared memory moves 480 KiB per 128 x 128 tile (operand reads 256, TMA writes of operands 64, dS 32, dQ staging in and out 128),
+// 3840 cycles at 128 B a cycle, beside 2560 cycles of MMA.  Measured at s = 8192, 32 / 8 heads, causal: 2173 us with one tile in flight and four
 // compute warps, 1251 us so, 1201 with dQ's columns handed back before its first quarter is sent.
 // reference semantics: the attention grad op of the reference, mindspeed/ops/csrc/cann/fusion_attention_v2.cpp:431-439.
 // =====================================================================================================================

@@ -186,51 +186,51 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1) gemm2_
       for (int i = 0; i < AHEAD; ++i) { sa[i] = scale_a(i); sb[i] = scale_b(i); }
       for (int kb0 = 0; kb0 < num_kb && alive; kb0 += AHEAD) {
 #pragma unroll
-       for (int u = 0; u < AHEAD; ++u) {                         // a slot keeps its register: moving it would wait for the load
-        const int kb = kb0 + u;
-        if (kb >= num_kb) break;
-        const float s = B_ROWWISE ? sa[u] : sa[u] * sb[u];
-        const uint64_t s2 = pack_f32x2(s, s);
-        sa[u] = scale_a(kb + AHEAD);
-        sb[u] = scale_b(kb + AHEAD);
-        if (B_ROWWISE && !mbar_wait(sfull_bar(slot), sphase, p.status, 0x531u)) { alive = false; break; }
-        if (!mbar_wait(tfull_bar(acc), acc_phase, p.status, 0x530u)) { alive = false; break; }
-        tc_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * PN + half * 128);
-        const uint32_t sb_row = smem_base + P_SC_OFF + (uint32_t)(slot * (PN * 4) + half * 512);
-        uint32_t r[2][16];                                       // the next 16 columns load while 16 are folded in
-        tmem_ld_32x16(t_row, r[0]);
+        for (int u = 0; u < AHEAD; ++u) {                         // a slot keeps its register: moving it would wait for the load
+          const int kb = kb0 + u;
+          if (kb >= num_kb) break;
+          const float s = B_ROWWISE ? sa[u] : sa[u] * sb[u];
+          const uint64_t s2 = pack_f32x2(s, s);
+          sa[u] = scale_a(kb + AHEAD);
+          sb[u] = scale_b(kb + AHEAD);
+          if (B_ROWWISE && !mbar_wait(sfull_bar(slot), sphase, p.status, 0x531u)) { alive = false; break; }
+          if (!mbar_wait(tfull_bar(acc), acc_phase, p.status, 0x530u)) { alive = false; break; }
+          tc_fence_after();
+          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * PN + half * 128);
+          const uint32_t sb_row = smem_base + P_SC_OFF + (uint32_t)(slot * (PN * 4) + half * 512);
+          uint32_t r[2][16];                                       // the next 16 columns load while 16 are folded in
+          tmem_ld_32x16(t_row, r[0]);
 #pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          tmem_ld_wait();
-          if (ch < 7) {
-            tmem_ld_32x16(t_row + (uint32_t)(16 * (ch + 1)), r[(ch + 1) & 1]);
-          } else {                                               // all of the accumulator is in registers
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(lead_tempty[acc]);
-          }
-          const uint32_t* v = r[ch & 1];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint64_t f0 = s2, f1 = s2;
-            if (B_ROWWISE) {
-              // broadcast: four columns' scales (volatile: hoisted loads cost registers that the accumulators need)
-              asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(f0), "=l"(f1) : "r"(sb_row + (uint32_t)((ch * 4 + j) * 16)));
-              f0 = mul_f32x2(s2, f0);
-              f1 = mul_f32x2(s2, f1);
+          for (int ch = 0; ch < 8; ++ch) {
+            tmem_ld_wait();
+            if (ch < 7) {
+              tmem_ld_32x16(t_row + (uint32_t)(16 * (ch + 1)), r[(ch + 1) & 1]);
+            } else {                                               // all of the accumulator is in registers
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_remote(lead_tempty[acc]);
             }
-            accum[ch * 8 + 2 * j] = fma_f32x2(f0, pack_u32x2(v[4 * j], v[4 * j + 1]), accum[ch * 8 + 2 * j]);
-            accum[ch * 8 + 2 * j + 1] = fma_f32x2(f1, pack_u32x2(v[4 * j + 2], v[4 * j + 3]), accum[ch * 8 + 2 * j + 1]);
+            const uint32_t* v = r[ch & 1];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint64_t f0 = s2, f1 = s2;
+              if (B_ROWWISE) {
+                // broadcast: four columns' scales (volatile: hoisted loads cost registers that the accumulators need)
+                asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(f0), "=l"(f1) : "r"(sb_row + (uint32_t)((ch * 4 + j) * 16)));
+                f0 = mul_f32x2(s2, f0);
+                f1 = mul_f32x2(s2, f1);
+              }
+              accum[ch * 8 + 2 * j] = fma_f32x2(f0, pack_u32x2(v[4 * j], v[4 * j + 1]), accum[ch * 8 + 2 * j]);
+              accum[ch * 8 + 2 * j + 1] = fma_f32x2(f1, pack_u32x2(v[4 * j + 2], v[4 * j + 3]), accum[ch * 8 + 2 * j + 1]);
+            }
           }
+          if (B_ROWWISE) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sempty_bar(slot));
+            if (++slot == PSC) { slot = 0; sphase ^= 1u; }
+          }
+          if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
         }
-        if (B_ROWWISE) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(sempty_bar(slot));
-          if (++slot == PSC) { slot = 0; sphase ^= 1u; }
-        }
-        if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
-       }
       }
       if (!alive) break;
       constexpr int CW = EPI == PEPI_BF16 ? 64 : 32;             // columns per 128-byte staging row

@@ -180,52 +180,52 @@ __global__ void __launch_bounds__(320, 1) gemm_fp8_blockscaled_kernel(const __gr
       for (int i = 0; i < AHEAD; ++i) { sa_q[i] = scale_a(i); sb_q[i] = scale_b(i); }
       for (int kb0 = 0; kb0 < num_kb && alive; kb0 += AHEAD) {
 #pragma unroll
-       for (int u = 0; u < AHEAD; ++u) {                   // a slot keeps its register: moving it would wait for the load
-        const int kb = kb0 + u;
-        if (kb >= num_kb) break;
-        const float sa = sa_q[u], sbs = sb_q[u];
-        sa_q[u] = scale_a(kb + AHEAD);
-        sb_q[u] = scale_b(kb + AHEAD);
-        if (!mbar_wait(tfull_bar(acc), acc_phase, p.status, 0x430u)) { alive = false; break; }
-        tc_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * FBN + cbase);
-        if (!p.b_scale_rowwise) {
-          const float s = sa * sbs;
+        for (int u = 0; u < AHEAD; ++u) {                   // a slot keeps its register: moving it would wait for the load
+          const int kb = kb0 + u;
+          if (kb >= num_kb) break;
+          const float sa = sa_q[u], sbs = sb_q[u];
+          sa_q[u] = scale_a(kb + AHEAD);
+          sb_q[u] = scale_b(kb + AHEAD);
+          if (!mbar_wait(tfull_bar(acc), acc_phase, p.status, 0x430u)) { alive = false; break; }
+          tc_fence_after();
+          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * FBN + cbase);
+          if (!p.b_scale_rowwise) {
+            const float s = sa * sbs;
 #pragma unroll
-          for (int c2 = 0; c2 < HC; c2 += 32) {
-            uint32_t r0[16], r1[16];                       // two 16-column loads in flight per wait
-            tmem_ld_32x16(t_row + (uint32_t)c2, r0);
-            tmem_ld_32x16(t_row + (uint32_t)(c2 + 16), r1);
-            tmem_ld_wait();
+            for (int c2 = 0; c2 < HC; c2 += 32) {
+              uint32_t r0[16], r1[16];                       // two 16-column loads in flight per wait
+              tmem_ld_32x16(t_row + (uint32_t)c2, r0);
+              tmem_ld_32x16(t_row + (uint32_t)(c2 + 16), r1);
+              tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              accum[c2 + j] = fmaf(s, __uint_as_float(r0[j]), accum[c2 + j]);
-              accum[c2 + 16 + j] = fmaf(s, __uint_as_float(r1[j]), accum[c2 + 16 + j]);
+              for (int j = 0; j < 16; ++j) {
+                accum[c2 + j] = fmaf(s, __uint_as_float(r0[j]), accum[c2 + j]);
+                accum[c2 + 16 + j] = fmaf(s, __uint_as_float(r1[j]), accum[c2 + 16 + j]);
+              }
+            }
+          } else {
+            const float* sbrow = p.sB + (long long)kb * ((long long)p.G * p.N) + ncol0 + cbase;
+#pragma unroll
+            for (int c2 = 0; c2 < HC; c2 += 32) {
+              uint32_t r0[16], r1[16];
+              tmem_ld_32x16(t_row + (uint32_t)c2, r0);
+              tmem_ld_32x16(t_row + (uint32_t)(c2 + 16), r1);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const int ca = c2 + j, cb = c2 + 16 + j;
+                const float sb0 = (n_blk * FBN + cbase + ca < p.N) ? __ldg(sbrow + ca) : 0.f;
+                const float sb1 = (n_blk * FBN + cbase + cb < p.N) ? __ldg(sbrow + cb) : 0.f;
+                accum[ca] = fmaf(sa * sb0, __uint_as_float(r0[j]), accum[ca]);
+                accum[cb] = fmaf(sa * sb1, __uint_as_float(r1[j]), accum[cb]);
+              }
             }
           }
-        } else {
-          const float* sbrow = p.sB + (long long)kb * ((long long)p.G * p.N) + ncol0 + cbase;
-#pragma unroll
-          for (int c2 = 0; c2 < HC; c2 += 32) {
-            uint32_t r0[16], r1[16];
-            tmem_ld_32x16(t_row + (uint32_t)c2, r0);
-            tmem_ld_32x16(t_row + (uint32_t)(c2 + 16), r1);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int ca = c2 + j, cb = c2 + 16 + j;
-              const float sb0 = (n_blk * FBN + cbase + ca < p.N) ? __ldg(sbrow + ca) : 0.f;
-              const float sb1 = (n_blk * FBN + cbase + cb < p.N) ? __ldg(sbrow + cb) : 0.f;
-              accum[ca] = fmaf(sa * sb0, __uint_as_float(r0[j]), accum[ca]);
-              accum[cb] = fmaf(sa * sb1, __uint_as_float(r1[j]), accum[cb]);
-            }
-          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(tempty_bar(acc));     // one arrival per warp: 256 on one barrier serialise
+          if (++acc == NACC) { acc = 0; acc_phase ^= 1u; }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tempty_bar(acc));     // one arrival per warp: 256 on one barrier serialise
-        if (++acc == NACC) { acc = 0; acc_phase ^= 1u; }
-       }
       }
       if (!alive) break;
       if (row_ok) {

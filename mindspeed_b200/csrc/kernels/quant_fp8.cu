@@ -11,7 +11,7 @@
 // Bound by memory: 2 bytes read and 1 (row or column) or 2 (both, block) written per bf16 element.  A CTA owns a 128 x 128 tile;
 // a thread owns 8 rows x 8 columns of it in registers, so that eight consecutive bytes of a row AND of a column leave one
 // thread: row bytes go straight to global memory, column bytes through a shared-memory transpose, both in whole 128-byte lines.
-// 4096 x 28672 bf16 (117 M elements, 470 MB): both forms 238 us, block form 174 us, where the PyTorch passes took 2.2 ms each; the IEEE
+// 4096 x 28672 bf16 (117 M elements, 470 MB): both forms 244 us, block form 178 us, where the PyTorch passes took 2.2 ms each; the IEEE
 // divisions keep it from the memory rate (72 us).
 // reference: mindspeed/te/pytorch/fp8/recipes/float8_block_scaling_recipe.py:15-26.
 #include "msb_common.cuh"

@@ -5,7 +5,7 @@
   fp8_grouped_gemm(xq, xs, wq, ws, counts)  expert-sorted rows; experts padded to 128-row tiles internally
   Fp8BlockwiseLinearFn                      y = x W^T with all three GEMMs in fp8:
         fprop   x  -> 1x128 along K ; W   -> 128x128            (K-major both)
-        dgrad   dy -> 1x128 along N ; W^T -> 128x128            (the transposed weight is quantised separately)
+        dgrad   dy -> 1x128 along N ; W^T -> 128x128            (on a GPU one pass writes the weight's form and its transpose)
         wgrad   dy^T, x^T -> 1x128 along the token dimension, both row-wise scaled, fp32 accumulation
   On CPU (or for shapes the kernel does not take) the fp32 reference of the same math is used, so the numerics of
   the recipe - not only its speed - are testable without a GPU.
